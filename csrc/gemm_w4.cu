@@ -56,7 +56,9 @@ struct W4Cfg {
   static constexpr bool kTiedX = !DUAL && NT <= 128;
   static constexpr int kSP = DUAL ? 2 : (NT <= 64 ? 3 : 2);        // slots in TMEM (DUAL: one per pipeline)
   static constexpr int kSX = DUAL ? 4 : (kTiedX ? kSP * kCPS / R : 2);      // activation stages
-  static constexpr int kSW = DUAL ? (NT == 64 ? 5 : 6) : (NT <= 64 ? 12 : (NT == 128 ? (R == 2 ? 10 : 8) : 8));
+  // (the narrow CTA's depth is even: with an odd one a slot would change pipelines with every use, and a pipeline ahead of a
+  // late copy of the other would take the slot's older phase, of equal parity, for its own)
+  static constexpr int kSW = DUAL ? (NT == 64 ? 4 : 6) : (NT <= 64 ? 12 : (NT == 128 ? (R == 2 ? 10 : 8) : 8));
   static constexpr int kAcc = (DUAL ? 2 : R) * NT;                 // accumulator columns (DUAL: one per pipeline)
   static_assert(kAcc + kSP * kCPS * 64 <= kTmemCols, "TMEM budget");
   static constexpr int kRingBytes = kSX * kXStage + kSW * kW4ChunkBytes;

@@ -48,8 +48,8 @@ namespace zse {
 
 constexpr int kDecWarps = 25;
 constexpr int kDecThreads = kDecWarps * 32;
-constexpr int kDecSX = 6;            // activation stages (INT4; INT8 chunks are twice as large: 5)
-constexpr int kDecSW = 5;            // weight chunks per pipeline ring (INT4; INT8: 3)
+constexpr int kDecSX = 6;            // activation stages (INT4; INT8 chunks are twice as large: 4)
+constexpr int kDecSW = 5;            // weight chunks per pipeline ring (INT4; INT8: 4)
 constexpr int kW8ChunkBytes = 16640; // INT8 chunk: 128 rows x 128 K int8 + 128 fp16 scales
 constexpr int kDecProducerWarp = 4;
 constexpr int kDecDqWarp0 = 5;
@@ -71,8 +71,12 @@ struct DecBars {
 
 template <int NT, bool W8 = false>
 struct DecCfg {
-  static constexpr int kSX = W8 ? 5 : kDecSX;
-  static constexpr int kSW = W8 ? 3 : kDecSW;
+  // Even and odd chunks of a pipeline have readers of their own.  In a ring of odd depth a slot changes readers with
+  // every use, and a reader that is one use ahead of a late copy takes the slot's older phase for its own (same parity).
+  // INT4: the weights of chunk c are waited for before the activations of step c + 1 are requested, which keeps the
+  // readers of an odd weight ring in order; the activation ring is even.  INT8 with 5 and 3 had neither and faulted.
+  static constexpr int kSX = W8 ? 4 : kDecSX;
+  static constexpr int kSW = W8 ? 4 : kDecSW;
   static constexpr int kChunk = W8 ? kW8ChunkBytes : kW4ChunkBytes;
   static constexpr int kXBytes = NT * 128;                  // one 64-wide K sub-tile of X
   static constexpr int kXStage = 2 * kXBytes;
@@ -80,9 +84,10 @@ struct DecCfg {
   static constexpr int kWRing = 2 * kSW * kChunk;
   static constexpr int kStageOff = kXRing + ((kWRing + 127) / 128) * 128;
   static constexpr int kBarsOff = kStageOff + kDecStageBytes;
-  static constexpr int kSmemBytes = kBarsOff + 1024 + 1024;   // barriers + alignment slack
+  static constexpr int kSmemWant = kBarsOff + 1024 + 1024;    // barriers + alignment slack
+  static constexpr int kSmemBytes = kSmemWant < 232448 ? kSmemWant : 232448;
   static constexpr int kGranules = NT / 8;                    // 8-column granules of the token dimension
-  static_assert(kSmemBytes <= 232448, "shared memory budget");
+  static_assert(kBarsOff + int(sizeof(DecBars)) <= kSmemBytes, "shared memory budget");
   // split plan: the receive area [S][2][ceil(G/S)][8][128] fp32 lies over both rings (S * ceil(G/S) <= G + S - 1)
   static_assert((kGranules + 7) * 2 * 8 * 128 * 4 <= kStageOff, "receive area of the split plan");
 };
@@ -837,7 +842,7 @@ gemm_w4_dec_kernel(const __grid_constant__ CUtensorMap tmap_x, const DecArgs a) 
   using Cfg = DecCfg<NT, W8>;
   constexpr int SX = Cfg::kSX, SW = Cfg::kSW;
   constexpr int kChunk = Cfg::kChunk;
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* x_ring = smem;                                        // [SX][2][NT*128]
   uint8_t* w_ring = smem + Cfg::kXRing;                          // [2][SW][8704]

@@ -193,6 +193,25 @@ def test_int8_weights_stay_eight_bits_wide(ops, ws, M, N, K):
     assert _rel(got, x[:M].float() @ wd.T) < 2e-3
 
 
+@pytest.mark.parametrize("M,N,K", [(32, 512, 18944), (17, 3584, 3584), (60, 37888, 896)])
+def test_int8_weight_rings_that_wrap_many_times(ops, ws, M, N, K):
+    """Eight segments of 18 steps, 112 CTAs of three or four, and 148 CTAs of seven: each run again and again, because what
+    is looked for (a slot read one use early) depends on which copy comes late."""
+    g = torch.Generator(device="cuda").manual_seed(N)
+    q = torch.randint(-127, 128, (N, K), dtype=torch.int8, device="cuda", generator=g)
+    s = (torch.rand(N, K // 128, device="cuda", generator=g) * 1e-4 + 1e-4).half()
+    w = ops.make_linear([{"dtype": "int8", "data": q, "scales": s, "shape": (N, K)}], K, 128)
+    dense = (q.float().view(N, K // 128, 128) * s.float()[..., None]).view(N, K)
+    x = (torch.randn(M, K, device="cuda", generator=g) * 0.5).half()
+    want = x.float() @ dense.T
+    out = torch.empty(M, N, dtype=torch.float16, device="cuda")
+    for _ in range(200):
+        ops.linear(w, x, M, out)
+    torch.cuda.synchronize()
+    ops.check()
+    assert _rel(out, want) < 2e-3, _rel(out, want)
+
+
 @pytest.mark.parametrize("M,I,K", [(9, 192, 512), (64, 1728, 1024), (150, 320, 256)])
 def test_int8_gate_up_with_swiglu(ops, ws, M, I, K):
     g, gd = _parts8(I, K, 3)

@@ -7,22 +7,27 @@ weights (a ring of SW chunks per pipeline); four epilogue warps take the accumul
 done.  Pipeline 1 may run out of chunks at a pair boundary (a last pair of one tile): its lanes then only hand the
 activation stages back.
 
-The model runs every role as a coroutine under a random scheduler - copies complete in any order, each lane's
-tcgen05.commit events in that lane's issue order - and checks at every barrier test that the parity answer equals the
+The model runs every role as a coroutine under a random scheduler - copies complete in any order (``late``: now and then
+one is overtaken by all that were issued after it), each lane's tcgen05.commit events in that lane's issue order - and checks at every barrier test that the parity answer equals the
 answer by phase index, that no barrier gets more arrivals than its phase expects, that ring slots and TMEM slots are
 never refilled under a reader, that accumulators are never overwritten before the epilogue has read them, and that
 every run ends.  No GPU is involved.
 """
+import os
 import random
+import re
 
 import pytest
 
 from test_attention_tc_pipeline_model import Bar
 
-SX, SW = 6, 5
+SOURCE = os.path.join(os.path.dirname(__file__), "..", "csrc", "gemm_w4_dec.cu")
+SX, SW = 6, 5                           # INT4
+RINGS = {"int4": (SX, SW), "int8": (4, 4)}
 
 
-def run(n_steps, ks, k_first, n_real1, seed):
+def run(n_steps, ks, k_first, n_real1, seed, rings=(SX, SW), late=False):
+    SX, SW = rings
     rnd = random.Random(seed)
     w_full = [[Bar(1) for _ in range(SW)] for _ in range(2)]
     w_empty = [[Bar(4) for _ in range(SW)] for _ in range(2)]
@@ -209,7 +214,9 @@ def run(n_steps, ks, k_first, n_real1, seed):
                 acc_state[key], acc_readers[key] = "full", 4
                 acc_full[key[0]][key[1]].arrive()
         elif c < 0.3 and copies:
-            copies.pop(rnd.randrange(len(copies))).arrive()
+            i = rnd.randrange(len(copies))
+            if not late or i > 0 or rnd.random() < 0.003:
+                copies.pop(i).arrive()
         elif live:
             i = rnd.choice(live)
             try:
@@ -244,3 +251,17 @@ def test_the_shapes_of_the_14b_layer():
             g0, g1 = total * cta // 148, total * (cta + 1) // 148
             if g1 > g0:
                 run(g1 - g0, ks, g0 % ks, g1 - g0, seed=cta)
+
+
+@pytest.mark.parametrize("kind", sorted(RINGS))
+def test_a_late_copy_is_not_taken_for_the_use_before_it(kind):
+    for seed in range(40):
+        run(28, 28, 0, 28, seed, RINGS[kind], late=True)
+        run(23, 9, 4, 14, seed, RINGS[kind], late=True)
+
+
+def test_the_rings_of_the_kernel_are_those_modelled():
+    text = open(SOURCE).read()
+    depth = {n: int(re.search(r"constexpr int kDec%s = (\d+);" % n, text).group(1)) for n in ("SX", "SW")}
+    assert (depth["SX"], depth["SW"]) == RINGS["int4"]
+    assert tuple(int(re.search(r"kS%s = W8 \? (\d+) : kDecS%s;" % (n, n), text).group(1)) for n in "XW") == RINGS["int8"]

@@ -2,19 +2,22 @@
 
 Roles of one CTA: a weight loader and an activation loader (rings of SW and SX stages), two MMA-issuing threads (chunks of
 even / odd index), two dequantisation groups of four warps (one per pipeline).  They meet at mbarriers tested by parity;
-the model runs them as coroutines under a random scheduler (copies complete in any order, each MMA thread's commits in
+the model runs them as coroutines under a random scheduler (copies complete in any order - ``late``: now and then one is
+overtaken by all that were issued after it - each MMA thread's commits in
 its own issue order) and checks, at every test, that the parity answer equals the answer by phase index, that no barrier
 ever receives more arrivals than its phase expects, that a ring stage is never refilled while a reader still needs it,
 and that every run ends.  No GPU is involved.
 """
+import os
 import random
+import re
 
 import pytest
 
 from test_attention_tc_pipeline_model import Bar
 
 
-def run(n_chunks, SW, SX, seed):
+def run(n_chunks, SW, SX, seed, late=False):
     rnd = random.Random(seed)
     w_full = [Bar(1) for _ in range(SW)]
     w_empty = [Bar(4) for _ in range(SW)]
@@ -107,7 +110,9 @@ def run(n_chunks, SW, SX, seed):
             p = rnd.choice([i for i in range(2) if pipes[i]])
             pipes[p].pop(0).arrive()
         elif c < 0.3 and copies:
-            copies.pop(rnd.randrange(len(copies))).arrive()
+            i = rnd.randrange(len(copies))
+            if not late or i > 0 or rnd.random() < 0.003:
+                copies.pop(i).arrive()
         elif live:
             i = rnd.choice(live)
             try:
@@ -119,8 +124,19 @@ def run(n_chunks, SW, SX, seed):
     assert len(done) == 8 and acc_ready.phase == 1
 
 
-@pytest.mark.parametrize("SW", [5, 6])
+@pytest.mark.parametrize("SW", [4, 6])
 @pytest.mark.parametrize("n_chunks", [1, 2, 3, 4, 5, 6, 7, 12, 16, 23])
 def test_narrow_cta_protocol(n_chunks, SW):
     for seed in range(25):
         run(n_chunks, SW, 4, seed)
+
+
+@pytest.mark.parametrize("SW", [4, 6])
+def test_a_late_copy_is_not_taken_for_the_use_before_it(SW):
+    for seed in range(60):
+        run(40, SW, 4, seed, late=True)
+
+
+def test_the_ring_of_the_kernel_is_one_of_those_modelled():
+    text = open(os.path.join(os.path.dirname(__file__), "..", "csrc", "gemm_w4.cu")).read()
+    assert re.search(r"kSW = DUAL \? \(NT == 64 \? (\d+) : (\d+)\)", text).groups() == ("4", "6")
