@@ -25,6 +25,10 @@ int zse_get_pdl(void);
 int zse_gemm_w4(const void* w_tiled, const void* x, int x_rows_cap, const void* bias, void* out, int M, int N, int K,
                 int ldo, int epilogue, int k_split, void* status, void* stream);
 int zse_gemm_w4_splits(int M, int N, int K, int k_split);
+// INT8 chunks (zse_repack_w8), same epilogues; gemm_pair.cu
+int zse_gemm_w8(const void* w_tiled, const void* x, int x_rows_cap, const void* bias, void* out, int M, int N, int K,
+                int ldo, int epilogue, int k_split, void* status, void* stream);
+int zse_gemm_w8_splits(int M, int N, int K, int k_split);
 // the launcher's plan for a call: out4 = {tiles per wide CTA, K splits, cluster size, CTA shape: 0 wide, 1 narrow,
 // -1 CUDA-core GEMV}
 void zse_gemm_w4_plan(int M, int N, int K, int epilogue, int k_split, int sm_count, int* out4);

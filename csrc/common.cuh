@@ -205,6 +205,15 @@ __device__ __forceinline__ void tc_commit(uint64_t* bar) {   // one thread
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// True in one lane of a converged warp.  A warp that issues tcgen05.mma walks its loop as a whole and lets one elected lane
+// issue: descriptors and TMEM addresses then live in uniform registers.  With a single lane in the loop every MMA pays for
+// moving them there (75 cycles an MMA in gemm_pair.cu, 25 this way).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // D[tmem] (+)= A[smem] * B[smem], kind::f16 (fp16 or bf16 inputs, fp32 accumulate); one thread.
 __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                         uint32_t accumulate) {

@@ -69,7 +69,7 @@ uint32_t* tp_push_state(const void* ctx, int rank_override);
 //              the tp rows in rank order and its fp32 residual row (the residual stream is sharded by rows during such
 //              a pass), normalises, and
 //   gather   - stores the fp16 row into `xg` on EVERY rank; the CTA that completes a block publishes the pass epoch
-//              in gflag[b] on every rank.  The column-parallel GEMM that consumes `xg` (gemm_w4.cu, activation
+//              in gflag[b] on every rank.  The column-parallel GEMM that consumes `xg` (gemm_pair.cu, activation
 //              producer) waits for the flags of the row blocks of its own token tile before its TMA loads: the gather
 //              is part of that GEMM's prologue, tile by tile.
 // The epoch lives in device memory (state[0], advanced by the last CTA of every reduce launch), so CUDA graphs
@@ -96,6 +96,12 @@ int tp_fill_sp_table(const void* ctx, int slot, bool multimem, int rank_override
 int gemv_w4_plan(int M, int N, int K, int epilogue, int sm_count, int want_split);
 int gemv_w4_launch(const void* w_tiled, const void* x, const void* bias, void* out, int M, int N, int K, int ldo,
                    int epilogue, int ks, cudaStream_t st);
+
+// Pairs of CTAs on 256 weight rows (gemm_pair.cu): INT4 or INT8 chunks, passes of more than 64 tokens, epilogues fp16, SwiGLU and
+// fp32 planes.  gemm_pair_planes: planes the last one writes.
+int gemm_pair_run(bool w8, const void* w_tiled, const void* x, int x_rows_cap, const void* bias, void* out, int M, int N,
+                  int K, int ldo, int epilogue, int want_split, const GatherWait* gather, Status* status, cudaStream_t st);
+int gemm_pair_planes(int M, int N, int K, int want_split);
 
 inline int pick_nt(int M) {
   if (M <= 16) return 16;

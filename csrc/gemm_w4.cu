@@ -93,7 +93,6 @@ struct W4Args {
   long long* timing;       // debug builds (ZSE_W4_TIMING): per-role cycle counters, else unused
   PushTable push;          // kEpiPushF16: where the partial tiles go (every rank's inbox over NVLink)
   SpTable sp;              // kEpiScatterF16: where the partial tiles go (the owner of each 64-row block)
-  GatherWait gather;       // the activations are a gathered buffer: wait for the row blocks of this CTA's token tile
 };
 
 __device__ __forceinline__ void multimem_st_v4(void* mc_ptr, const uint4& v) {
@@ -111,35 +110,6 @@ __device__ __forceinline__ void red_add_relaxed_sys(uint32_t* p, uint32_t v) {
 __device__ __forceinline__ void red_add_release_sys(uint32_t* p, uint32_t v) {
   asm volatile("red.release.sys.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ uint32_t w4_ld_acquire_sys(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-// All-gather in the prologue: the rows of token tile [t0, t0 + nt) were written into this GPU's memory by their
-// owners (other GPUs, plain or multicast stores); a row block is complete when its flag holds the pass epoch.  One
-// thread waits (bounded), then orders those writes before the TMA loads it is about to issue (async proxy).
-__device__ __forceinline__ bool gather_wait_tile(const GatherWait& g, int t0, int nt, int M, volatile int* abort_flag,
-                                                 Status* st) {
-  const uint32_t want = *reinterpret_cast<const volatile uint32_t*>(g.epoch);
-  bool ok = true;
-  for (int t = t0; t < t0 + nt && t < M && ok; t += kSpRowBlock) {
-    const uint32_t* f = g.flags + t / kSpRowBlock;
-    if (w4_ld_acquire_sys(f) == want) continue;
-    SpinClock clk;
-    while (w4_ld_acquire_sys(f) != want) {
-      if (clk.expired(0x3F) || ((clk.spins & 0x3F) == 0 && *abort_flag)) {
-        report(st, kPeerTimeout, 36, unsigned(t / kSpRowBlock));
-        *abort_flag = 1;
-        ok = false;
-        break;
-      }
-    }
-  }
-  asm volatile("fence.proxy.async;" ::: "memory");
-  return ok;
-}
-
 // Nibble order inside every 32-bit word of a chunk (fixed by repack_w4): positions 0..7 hold the K elements
 // e0,e2,e4,e6,e1,e3,e5,e7 so that masking with 0x000f000f yields the adjacent pair (e0,e1) as a half2.
 __device__ __forceinline__ void dequant_word(uint32_t w, __half2 s2, __half2 z2, uint32_t* out4) {
@@ -445,10 +415,7 @@ gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Args a) {
       int issued = 0, s = 0;
       uint32_t ph = 1;
       pdl_wait();                                        // the activations come from the previous kernel
-      bool gathered = true;
-      if (a.gather.flags != nullptr)
-        gathered = gather_wait_tile(a.gather, blockIdx.y * NT, NT, a.M, abort_flag, a.status);
-      for (int kk = 0; kk < n_k && gathered; ++kk) {
+      for (int kk = 0; kk < n_k; ++kk) {
         if (kk >= SX) {
           // tied: the commit that ends the pair holding this stage's last chunk frees the stage as well
           uint64_t* freed = kTied ? &bars->pair_done[s / (CPS / R)] : &bars->x_empty[s];
@@ -827,12 +794,13 @@ static int launch_w4(const CUtensorMap& tx, const W4Args& a, dim3 grid, cudaStre
 
 template <int NT, int R, bool DUAL = false>
 static int launch_w4_epi(int epilogue, const CUtensorMap& tx, const W4Args& a, dim3 grid, cudaStream_t st) {
-  if (epilogue == kEpiF16) return launch_w4<NT, R, kEpiF16, DUAL>(tx, a, grid, st);
-  if (epilogue == kEpiSwiGLU) return launch_w4<NT, R, kEpiSwiGLU, DUAL>(tx, a, grid, st);
-  if (epilogue == kEpiPartialF32) return launch_w4<NT, R, kEpiPartialF32, DUAL>(tx, a, grid, st);
   if (epilogue == kEpiPushF16) return launch_w4<NT, R, kEpiPushF16, DUAL>(tx, a, grid, st);
-  if constexpr (NT >= 128) {         // the row-block exchange is for passes of many rows
+  if constexpr (NT >= 128) {         // more than 64 rows: only the exchanges with other ranks come here (gemm_pair.cu)
     if (epilogue == kEpiScatterF16) return launch_w4<NT, R, kEpiScatterF16, DUAL>(tx, a, grid, st);
+  } else {
+    if (epilogue == kEpiF16) return launch_w4<NT, R, kEpiF16, DUAL>(tx, a, grid, st);
+    if (epilogue == kEpiSwiGLU) return launch_w4<NT, R, kEpiSwiGLU, DUAL>(tx, a, grid, st);
+    if (epilogue == kEpiPartialF32) return launch_w4<NT, R, kEpiPartialF32, DUAL>(tx, a, grid, st);
   }
   return ZSE_ERR_SHAPE;
 }
@@ -937,6 +905,9 @@ static int run_gemm_w4(const void* w_tiled, const void* x, int x_rows_cap, const
     if (gks > 0)
       return gemv_w4_launch(w_tiled, x, bias, out, M, N, K, ldo, epilogue, gks, reinterpret_cast<cudaStream_t>(stream));
   }
+  if (push == nullptr && sp == nullptr && M > 64)       // (a K split of a fused epilogue is a plan of the kernels below)
+    return gemm_pair_run(false, w_tiled, x, x_rows_cap, bias, out, M, N, K, ldo, epilogue, k_split, gather,
+                         reinterpret_cast<Status*>(status), reinterpret_cast<cudaStream_t>(stream));
   const int k_stages = K / kW4StageK;
   int R = 1, ks = 1, cluster = 1, dual = 0;
   plan_w4(M, N, K, epilogue, sm_count, k_split, &R, &ks, &cluster, &dual);
@@ -948,11 +919,9 @@ static int run_gemm_w4(const void* w_tiled, const void* x, int x_rows_cap, const
   CUtensorMap tx;
   if (int rc = get_tmap(x, uint64_t(max(x_rows_cap, M)), uint64_t(K), uint32_t(nt), &tx)) return rc;
   W4Args a{reinterpret_cast<const uint8_t*>(w_tiled), reinterpret_cast<const __half*>(bias), out, M, N, K, ldo,
-           k_stages, spp, cluster, reinterpret_cast<Status*>(status), g_w4_timing, PushTable{}, SpTable{},
-           GatherWait{nullptr, nullptr}};
+           k_stages, spp, cluster, reinterpret_cast<Status*>(status), g_w4_timing, PushTable{}, SpTable{}};
   if (push != nullptr) a.push = *push;
   if (sp != nullptr) a.sp = *sp;
-  a.gather = gather != nullptr ? *gather : GatherWait{nullptr, nullptr};
   dim3 grid(n_tiles / R, (M + nt - 1) / nt, ks);
   if (ctas_out != nullptr) *ctas_out = int(grid.x * grid.y * grid.z);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -1083,6 +1052,7 @@ extern "C" int zse_gemm_w4_splits(int M, int N, int K, int k_split) {
     const int gks = gemv_w4_plan(M, N, K, kEpiPartialF32, sm_count, k_split);
     if (gks > 0) return gks;
   }
+  if (M > 64) return gemm_pair_planes(M, N, K, k_split);
   int R = 1, ks = 1, cluster = 1, dual = 0;
   plan_w4(M, N, K, kEpiPartialF32, sm_count, k_split, &R, &ks, &cluster, &dual);
   const int k_stages = K / kW4StageK;

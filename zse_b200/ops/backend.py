@@ -687,8 +687,8 @@ class CudaOps(TorchOps):
             out = torch.empty(n_tiles * (K // 128) * 8704, dtype=torch.uint8, device=self.device)
             n.repack_w4(packed, scales, zeros, out, N, K, inter)
             return LinearWeight("w4t", N, K, out, b, swiglu, out.numel())
-        # INT8 (symmetric groups of 128): kept 8 bits wide, tiled for the decode kernel.  Passes of more than 64 tokens
-        # expand the tensor into a scratch buffer that all layers share and run the fp16 GEMM on it.
+        # INT8 (symmetric groups of 128): kept 8 bits wide, tiled for the decode kernel and (more than 64 tokens) the
+        # paired kernel of INT4.
         w8_ok = (K % 128 == 0 and group_size == 128 and all(p["dtype"] == "int8" and "scales" in p for p in parts)
                  and self.int8_resident)
         if swiglu and w8_ok:
@@ -727,8 +727,7 @@ class CudaOps(TorchOps):
                 self.n.gemm_w8_dec(w.data, x, cap, w.bias, out, M, w.N, w.K, out.stride(0), EPI_F16, self.dec_ws,
                                    self.status.ptr)
             else:
-                self.n.gemm_f16(self._w8_dense(w), w.N, x, cap, w.bias, out, M, w.N, w.K, out.stride(0), EPI_F16, 1,
-                                self.status.ptr)
+                self.n.gemm_w8(w.data, x, cap, w.bias, out, M, w.N, w.K, out.stride(0), EPI_F16, 0, self.status.ptr)
         elif (w.kind == "w4t" and (self.dec_mode & 4) and M <= 64 and out.stride(0) % 8 == 0
                 and self.n.gemm_w4_dec_supported(M, w.N, w.K, EPI_F16)):
             self.n.gemm_w4_dec(w.data, x, cap, w.bias, out, M, w.N, w.K, out.stride(0), EPI_F16, self.dec_ws,
@@ -754,6 +753,8 @@ class CudaOps(TorchOps):
                     and self.n.gemm_w4_dec_supported(M, w.N, w.K, EPI_SWIGLU)):
                 self.n.gemm_w8_dec(w.data, x, cap, None, out, M, w.N, w.K, out.stride(0), EPI_SWIGLU, self.dec_ws,
                                    self.status.ptr)
+            elif not gelu:
+                self.n.gemm_w8(w.data, x, cap, None, out, M, w.N, w.K, out.stride(0), EPI_SWIGLU, 0, self.status.ptr)
             else:
                 gu = torch.empty(M, w.N, dtype=torch.float16, device=self.device) if tmp is None else tmp
                 self.n.gemm_f16(self._w8_dense(w), w.N, x, cap, None, gu, M, w.N, w.K, gu.stride(0), EPI_F16, 1,
@@ -790,9 +791,14 @@ class CudaOps(TorchOps):
                 self.n.gemm_w8_dec(w.data, x, cap, None, partials, M, w.N, w.K, w.N, EPI_PARTIAL, self.dec_ws,
                                    self.status.ptr)
                 return 1
-            dense = self._w8_dense(w)
-            dw = LinearWeight("f16", w.N, w.K, dense, None, False, 0)
-            return self.linear_partial(dw, x, M, partials, k_split, x_cap)
+            ks = 0 if k_split is None else k_split
+            planes = self.n.gemm_w8_splits(M, w.N, w.K, ks)
+            if planes > partials.shape[0]:
+                ks = partials.shape[0]
+                planes = self.n.gemm_w8_splits(M, w.N, w.K, ks)
+            self.n.gemm_w8(w.data, x, cap, None, partials, M, w.N, w.K, partials.stride(1), EPI_PARTIAL, ks,
+                           self.status.ptr)
+            return planes
         if w.kind == "w4t":
             ks = 0 if k_split is None else min(k_split, partials.shape[0])
             planes = self.n.gemm_w4_splits(M, w.N, w.K, ks)

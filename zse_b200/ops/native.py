@@ -115,6 +115,9 @@ _SIGS = {
     "zse_gemm_w4": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                             c_void_p, c_void_p]),
     "zse_gemm_w4_splits": (c_int, [c_int, c_int, c_int, c_int]),
+    "zse_gemm_w8": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
+                            c_void_p, c_void_p]),
+    "zse_gemm_w8_splits": (c_int, [c_int, c_int, c_int, c_int]),
     "zse_gemm_w4_dec": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                 c_void_p, c_void_p, c_void_p]),
     "zse_gemm_w4_dec_qkv_rope": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
@@ -434,6 +437,16 @@ def gemm_w4_dec_plan(N, K, epilogue, sm_count):
 def gemm_f16(w, w_rows, x, x_rows_cap, bias, out, M, N, K, ldo, epilogue, k_split, status):
     _ck(load().zse_gemm_f16(_p(w), w_rows, _p(x), x_rows_cap, _p(bias), _p(out), M, N, K, ldo, epilogue, k_split,
                             status, _stream()), "gemm_f16")
+
+
+def gemm_w8(w_tiled, x, x_rows_cap, bias, out, M, N, K, ldo, epilogue, k_split, status):
+    """``gemm_w4`` for INT8 weights tiled by ``repack_w8``: passes of more than 64 tokens."""
+    _ck(load().zse_gemm_w8(_p(w_tiled), _p(x), x_rows_cap, _p(bias), _p(out), M, N, K, ldo, epilogue, k_split,
+                           status, _stream()), "gemm_w8")
+
+
+def gemm_w8_splits(M, N, K, k_split) -> int:
+    return load().zse_gemm_w8_splits(M, N, K, k_split)
 
 
 def gemm_w4_splits(M, N, K, k_split) -> int:
