@@ -277,37 +277,39 @@ gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Args a) {
       }
     } else if (warp == 1 || warp == kIssuer1) {
       const int p = warp == 1 ? 0 : 1;
-      if (lane == 0) {
-        constexpr uint32_t idesc = make_idesc_f16(kTileN, NT);
-        const uint64_t desc0 = make_desc_sw128(smem_u32(x_ring));
-        const uint32_t at = a_base + p * 64, dt = tmem + p * NT;
-        uint32_t aph = 0;
-        for (int u = p; u < n_units; u += 2) {
-          const int sx = u % SX;
-          TICK(tx);
-          if (!ZSE_W4_ISSUER_WAIT(&bars->x_full[sx], (u / SX) & 1, abort_flag, a.status, 3, u)) break;
-          ACC(0, tx);
-          TICK(ta);
-          if (!ZSE_W4_ISSUER_WAIT(&bars->a_ready[p], aph, abort_flag, a.status, 4, u)) break;
-          ACC(1, ta);
-          TICK(ti);
-          tc_fence_after_sync();
+      constexpr uint32_t idesc = make_idesc_f16(kTileN, NT);
+      const uint64_t desc0 = make_desc_sw128(smem_u32(x_ring));
+      const uint32_t at = a_base + p * 64, dt = tmem + p * NT;
+      uint32_t aph = 0;
+      for (int u = p; u < n_units; u += 2) {
+        const int sx = u % SX;
+        TICK(tx);
+        if (!__all_sync(0xffffffffu, ZSE_W4_ISSUER_WAIT(&bars->x_full[sx], (u / SX) & 1, abort_flag, a.status, 3, u))) break;
+        ACC(0, tx);
+        TICK(ta);
+        if (!__all_sync(0xffffffffu, ZSE_W4_ISSUER_WAIT(&bars->a_ready[p], aph, abort_flag, a.status, 4, u))) break;
+        ACC(1, ta);
+        TICK(ti);
+        tc_fence_after_sync();
+        const uint64_t bd = desc0 + uint64_t((sx * Cfg::kXStage) >> 4);
+        if (elect_one()) {
           // slot p was refilled for this chunk only after the MMAs of chunk u-2 had completed, so the activation
           // stage that chunk used is free as well
 #ifndef ZSE_W4_EARLY_X
           if (u >= 2) mbar_arrive(&bars->x_empty[(u - 2) % SX]);
 #endif
-          const uint64_t bd = desc0 + uint64_t((sx * Cfg::kXStage) >> 4);
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             umma_ts(dt, at + j * 8, bd + uint64_t((j >> 2) * (Cfg::kXBytes >> 4) + (j & 3) * 2), idesc,
                     (u >= 2) || (j != 0));
           tc_commit(&bars->pair_done[p]);
-          aph ^= 1;
-          ACC(2, ti);
         }
-        tc_commit(&bars->acc_ready);
+        __syncwarp();
+        aph ^= 1;
+        ACC(2, ti);
       }
+      if (elect_one()) tc_commit(&bars->acc_ready);
+      __syncwarp();
     } else {
       const int q = warp & 3;                  // TMEM lane quarter this warp may touch
       const int p = (warp - 2) >> 2;           // pipeline = dequant group

@@ -14,7 +14,8 @@
 //    pipeline is worked by two lanes (even and odd K stages), and a lane is a closed loop of its own: a dequant group
 //    of four warps, one TMEM operand slot, one MMA-issuing warp and one accumulator.  Measured on B200, a thread that
 //    issues tcgen05.mma back to back gets one through every ~85 cycles (M 128, N 64, K 16, A in TMEM) whatever else
-//    it executes, while the tensor pipe needs 32: four issuing threads, one per scheduler, are what fills the pipe.
+//    it executes, while the tensor pipe needs 32 (a converged warp with an elected lane does better, see elect_one): four
+//    issuing warps, one per scheduler, are what fills the pipe.
 //      warps 0-3   MMA issuers of lane (pipeline p, parity s) (tcgen05.mma, A = dequantised weights in TMEM, B =
 //                  activations in shared memory); the two accumulators of a tile are added in the epilogue,
 //      warp 4      producer: bulk TMA of the weight chunks (one ring per pipeline), tiled TMA of the activations,
@@ -64,7 +65,6 @@ struct DecBars {
   uint64_t x_full[kDecSX], x_empty[kDecSX];
   uint64_t a_ready[2][2], slot_free[2][2];
   uint64_t acc_full[2][2], acc_empty[2][2];
-  uint64_t bdesc[kDecSX][8];     // activation descriptors of every (stage, K step): the MMA issuers only load them
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -270,34 +270,6 @@ __device__ __forceinline__ int dec_range_begin(const DecArgs& a, int c, int n_ct
     return pair * a.k_stages + int((long long)seg * a.k_stages / a.split);
   }
   return int((long long)c * a.total_steps / n_cta);
-}
-
-// Eight tcgen05.mma of one 128 x 128 chunk, back to back.  The issuing thread shares its scheduler with five busy
-// warps and gets an issue slot only every ten to thirty cycles, so what counts is the number of instructions it
-// executes per chunk: the eight activation descriptors of a stage come out of a table in shared memory (four 16-byte
-// loads), the eight TMEM operand addresses are loop-invariant registers, the predicate is set twice.
-__device__ __forceinline__ void dec_mma_chunk(uint32_t dt, const uint32_t (&at)[8], const uint64_t* bdesc_stage,
-                                              uint32_t idesc, uint32_t accumulate_first) {
-  const ulonglong2* tab = reinterpret_cast<const ulonglong2*>(bdesc_stage);
-  const ulonglong2 d01 = tab[0], d23 = tab[1], d45 = tab[2], d67 = tab[3];
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p, t;\n\t"
-      "setp.ne.b32 p, %17, 0;\n\t"
-      "setp.eq.b32 t, %18, %18;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %9, %18, p;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%2], %10, %18, t;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%3], %11, %18, t;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%4], %12, %18, t;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%5], %13, %18, t;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%6], %14, %18, t;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%7], %15, %18, t;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%8], %16, %18, t;\n\t"
-      "}" ::"r"(dt),
-      "r"(at[0]), "r"(at[1]), "r"(at[2]), "r"(at[3]), "r"(at[4]), "r"(at[5]), "r"(at[6]), "r"(at[7]), "l"(d01.x),
-      "l"(d01.y), "l"(d23.x), "l"(d23.y), "l"(d45.x), "l"(d45.y), "l"(d67.x), "l"(d67.y), "r"(accumulate_first),
-      "r"(idesc)
-      : "memory");
 }
 
 // Barriers of the threads that run an epilogue together: 128 (the four epilogue warps) or 640 (with the sixteen dequant
@@ -911,15 +883,6 @@ gemm_w4_dec_kernel(const __grid_constant__ CUtensorMap tmap_x, const DecArgs a) 
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
   }
-  if (threadIdx.x == 32) {
-    // the start-address field counts 16-byte units: a K step of 16 halfs is +2, the second 64-wide K sub-tile of a
-    // stage is +kXBytes/16
-    const uint64_t desc0 = make_desc_sw128(smem_u32(x_ring));
-    for (int st = 0; st < SX; ++st)
-      for (int j = 0; j < 8; ++j)
-        bars->bdesc[st][j] =
-            desc0 + uint64_t(((st * Cfg::kXStage) >> 4) + (j >> 2) * (Cfg::kXBytes >> 4) + (j & 3) * 2);
-  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -934,12 +897,13 @@ gemm_w4_dec_kernel(const __grid_constant__ CUtensorMap tmap_x, const DecArgs a) 
     // steps sub, sub + 2, ... of the CTA; waits are polled without the suspend hint (its wake-up is on the critical
     // path); every index is carried along, nothing is divided
     const int p = warp >> 1, sub = warp & 1;
-    if (lane == 0) {
+    {
       constexpr uint32_t idesc = make_idesc_f16(kTileN, NT);
-      const uint32_t acc = tmem + (2 * p + sub) * 64;
-      uint32_t at[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) at[j] = tmem + 256 + (2 * p + sub) * 64 + j * 8;
+      const uint32_t acc = tmem + (2 * p + sub) * 64, at = tmem + 256 + (2 * p + sub) * 64;
+      // the start-address field counts 16-byte units: a K step of 16 halfs is +2, the second 64-wide K sub-tile of a
+      // stage is +kXBytes/16
+      const uint64_t desc0 = make_desc_sw128(smem_u32(x_ring));
+      auto all = [](bool ok) { return __all_sync(0xffffffffu, ok) != 0; };
       const int my_steps = p == 0 ? n_steps : n_real1;
       int k = k_first + sub, item = 0, cur_item = -1, uses = 0;
       while (k >= ks) {
@@ -951,26 +915,32 @@ gemm_w4_dec_kernel(const __grid_constant__ CUtensorMap tmap_x, const DecArgs a) 
       int s = sub;
       for (; s < my_steps; s += 2) {
         DTICK(tx);
-        if (!mbar_wait_spin(&bars->x_full[st], xph, abort_flag, a.status, 3, s)) break;
+        if (!all(mbar_wait_spin(&bars->x_full[st], xph, abort_flag, a.status, 3, s))) break;
         DACC(0, tx);
         const bool first = item != cur_item;             // this lane's first chunk of a tile pair
         if (first) {
-          if (uses > 0 && !mbar_wait_spin(&bars->acc_empty[p][sub], (uses - 1) & 1, abort_flag, a.status, 4, item))
+          if (uses > 0 &&
+              !all(mbar_wait_spin(&bars->acc_empty[p][sub], (uses - 1) & 1, abort_flag, a.status, 4, item)))
             break;
           cur_item = item;
         }
         DTICK(ta);
-        if (!mbar_wait_spin(&bars->a_ready[p][sub], aph, abort_flag, a.status, 5, s)) break;
+        if (!all(mbar_wait_spin(&bars->a_ready[p][sub], aph, abort_flag, a.status, 5, s))) break;
         DACC(1, ta);
         DTICK(ti);
         aph ^= 1;
         tc_fence_after_sync();
-        dec_mma_chunk(acc, at, bars->bdesc[st], idesc, first ? 0u : 1u);
-        tc_commit(&bars->slot_free[p][sub]);
-        if (k + 2 >= ks || s + 2 >= n_steps) {             // this lane's last chunk of the pair
-          tc_commit(&bars->acc_full[p][sub]);
-          ++uses;
+        const bool last = k + 2 >= ks || s + 2 >= n_steps;   // this lane's last chunk of the pair
+        const uint64_t bd = desc0 + uint64_t((st * Cfg::kXStage) >> 4);
+        if (elect_one()) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            umma_ts(acc, at + j * 8, bd + uint64_t((j >> 2) * (Cfg::kXBytes >> 4) + (j & 3) * 2), idesc, j > 0 || !first);
+          tc_commit(&bars->slot_free[p][sub]);
+          if (last) tc_commit(&bars->acc_full[p][sub]);
         }
+        __syncwarp();
+        if (last) ++uses;
         DACC(2, ti);
         k += 2;
         while (k >= ks) {
@@ -984,10 +954,10 @@ gemm_w4_dec_kernel(const __grid_constant__ CUtensorMap tmap_x, const DecArgs a) 
         }
       }
       // no second tile in the rest of the range (pipeline 1 only): hand the stages back
-      if (!*abort_flag) {
+      if (all(!*abort_flag)) {
         for (; s < n_steps; s += 2) {
-          if (!mbar_wait_spin(&bars->x_full[st], xph, abort_flag, a.status, 3, s)) break;
-          mbar_arrive(&bars->x_empty[st]);
+          if (!all(mbar_wait_spin(&bars->x_full[st], xph, abort_flag, a.status, 3, s))) break;
+          if (lane == 0) mbar_arrive(&bars->x_empty[st]);
           st += 2;
           if (st >= SX) {
             st -= SX;
