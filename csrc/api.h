@@ -30,7 +30,7 @@ int zse_gemm_w8(const void* w_tiled, const void* x, int x_rows_cap, const void* 
                 int ldo, int epilogue, int k_split, void* status, void* stream);
 int zse_gemm_w8_splits(int M, int N, int K, int k_split);
 // the launcher's plan for a call: out4 = {tiles per wide CTA, K splits, cluster size, CTA shape: 0 wide, 1 narrow,
-// -1 CUDA-core GEMV}
+// -1 gemm_w4_small.cu}
 void zse_gemm_w4_plan(int M, int N, int K, int epilogue, int k_split, int sm_count, int* out4);
 // ---- gemm_w4_dec.cu -----------------------------------------------------------------------------------------
 // Decode-sized INT4 GEMM (M <= 64): one persistent CTA per SM over an even split of the weight stream.

@@ -14,7 +14,8 @@ constexpr int kGemmThreads = 320;    // fp16 kernel: warp 0 producer, warp 1 MMA
 
 enum Epilogue : int { kEpiF16 = 0, kEpiSwiGLU = 1, kEpiPartialF32 = 2, kEpiPushF16 = 3, kEpiScatterF16 = 4,
                      kEpiRelu2 = 5 /* bfloat16: store the square of relu */,
-                     kEpiGlu = 6 /* bfloat16: gated activation of 64 gate rows and their 64 up rows per tile */ };
+                     kEpiGlu = 6 /* bfloat16: gated activation of 64 gate rows and their 64 up rows per tile */,
+                     kEpiQkvRope = 7 /* gemm_w4_small.cu: a tile is a head; rotation, K/V rows into the paged cache */ };
 
 struct GemmArgs {
   const uint8_t* w;        // W4: tiled chunks [n_tiles][k_stages][8704]; F16: unused (tensor map)
@@ -91,11 +92,19 @@ struct GatherWait {
 };
 int tp_fill_sp_table(const void* ctx, int slot, bool multimem, int rank_override, SpTable* out);
 
-// CUDA-core path for one or two tokens (gemv_w4.cu).  gemv_w4_plan returns the number of K splits (fp32 planes) the
-// GEMV would use, or 0 when the tensor-core kernel should run instead.
-int gemv_w4_plan(int M, int N, int K, int epilogue, int sm_count, int want_split);
-int gemv_w4_launch(const void* w_tiled, const void* x, const void* bias, void* out, int M, int N, int K, int ldo,
-                   int epilogue, int ks, cudaStream_t st);
+// Up to 8 tokens on INT4 chunks (gemm_w4_small.cu); epilogues fp16, SwiGLU, fp32 planes and kEpiQkvRope (N = (nh + 2 nkv) * 128).
+// gemm_w4_small_planes: planes the third writes.
+struct SmallRope {
+  const int* positions;        // [M]
+  const long long* slots;      // [M] cache slot = block * block_size + offset; -1 = do not store
+  const float2* cos_sin;       // [max_position][64] {cos, sin} of position * inv_freq[i]
+  __half* kv_layer;            // [blocks][2][nkv][block_size][128]
+  int nh, nkv, block_size, max_position;
+};
+bool gemm_w4_small_takes(int M, int K);
+int gemm_w4_small_planes(int N, int K, int want_split);
+int gemm_w4_small_run(const void* w_tiled, const void* x, const void* bias, void* out, int M, int N, int K, int ldo,
+                      int epilogue, int want_split, const SmallRope* rope, cudaStream_t st);
 
 // Pairs of CTAs on 256 weight rows (gemm_pair.cu): INT4 or INT8 chunks, passes of more than 64 tokens, epilogues fp16, SwiGLU and
 // fp32 planes.  gemm_pair_planes: planes the last one writes.

@@ -808,7 +808,7 @@ static int launch_w4_epi(int epilogue, const CUtensorMap& tx, const W4Args& a, d
 }
 
 // 0 = the planner decides, 1 = wide CTAs only, 2 = narrow (two per SM) CTAs wherever they are allowed;
-// adding 4 keeps one- and two-token calls on the tensor cores instead of the CUDA-core GEMV
+// adding 4 keeps calls of up to 8 tokens on the kernels of this file instead of gemm_w4_small.cu
 static int g_w4_mode = 0;
 
 // How the launcher tiles a problem: weight tiles per CTA (R) and K splits (ks).  Measured on B200: a tcgen05.mma of
@@ -889,6 +889,13 @@ extern "C" void zse_gemm_w4_set_timing(void* dev_buffer) { g_w4_timing = reinter
 // Tuning hook: 0 = planner decides between wide and narrow CTAs, 1 = wide only, 2 = narrow wherever allowed.
 extern "C" void zse_gemm_w4_set_mode(int mode) { zse::g_w4_mode = mode; }
 
+// Up to 8 tokens: gemm_w4_small.cu, unless a tuning mode or a cluster along K asks for a CTA of this file.  Measured (B200, cold
+// L2, this file -> that one), 5 tokens: 7B gate/up 32.8 -> 23.5 us, down 21.5 -> 16.4, QKV 16.4 -> 12.3; a variant for 16 tokens
+// lost (gate/up 32.8 -> 41.8 us: twice the products, fewer warps for its registers).
+static bool takes_small(int M, int K, int epilogue, int k_split) {
+  return g_w4_mode == 0 && gemm_w4_small_takes(M, K) && (epilogue == kEpiPartialF32 || k_split <= 0);
+}
+
 static int run_gemm_w4(const void* w_tiled, const void* x, int x_rows_cap, const void* bias, void* out, int M, int N,
                        int K, int ldo, int epilogue, int k_split, void* status, void* stream, const PushTable* push,
                        int* ctas_out, const SpTable* sp = nullptr, const GatherWait* gather = nullptr) {
@@ -902,11 +909,9 @@ static int run_gemm_w4(const void* w_tiled, const void* x, int x_rows_cap, const
     if (sm_count <= 0) sm_count = 148;
   }
   if ((sp != nullptr || gather != nullptr) && M <= 64) return ZSE_ERR_SHAPE;   // wide CTAs (128 / 256 tokens) only
-  if (!(g_w4_mode & 4) && push == nullptr) {
-    const int gks = gemv_w4_plan(M, N, K, epilogue, sm_count, k_split);
-    if (gks > 0)
-      return gemv_w4_launch(w_tiled, x, bias, out, M, N, K, ldo, epilogue, gks, reinterpret_cast<cudaStream_t>(stream));
-  }
+  if (push == nullptr && takes_small(M, K, epilogue, k_split))
+    return gemm_w4_small_run(w_tiled, x, bias, out, M, N, K, ldo, epilogue, k_split, nullptr,
+                             reinterpret_cast<cudaStream_t>(stream));
   if (push == nullptr && sp == nullptr && M > 64)       // (a K split of a fused epilogue is a plan of the kernels below)
     return gemm_pair_run(false, w_tiled, x, x_rows_cap, bias, out, M, N, K, ldo, epilogue, k_split, gather,
                          reinterpret_cast<Status*>(status), reinterpret_cast<cudaStream_t>(stream));
@@ -1030,15 +1035,12 @@ extern "C" int zse_gemm_w4_max_clusters(int narrow, int cluster) {
 }
 
 // What the launcher would do for these arguments: out4 = {weight tiles per wide CTA, K splits, cluster size along K,
-// CTA shape (0 wide, 1 narrow)}; -1 in out4[3] = CUDA-core GEMV.
+// CTA shape (0 wide, 1 narrow)}; -1 in out4[3] = gemm_w4_small.cu.
 extern "C" void zse_gemm_w4_plan(int M, int N, int K, int epilogue, int k_split, int sm_count, int* out4) {
   if (sm_count <= 0) sm_count = 148;
-  if (!(g_w4_mode & 4)) {
-    const int gks = gemv_w4_plan(M, N, K, epilogue, sm_count, k_split);
-    if (gks > 0) {
-      out4[0] = 1, out4[1] = gks, out4[2] = 1, out4[3] = -1;
-      return;
-    }
+  if (takes_small(M, K, epilogue, k_split)) {
+    out4[0] = 1, out4[1] = epilogue == kEpiPartialF32 ? gemm_w4_small_planes(N, K, k_split) : 1, out4[2] = 1, out4[3] = -1;
+    return;
   }
   plan_w4(M, N, K, epilogue, sm_count, k_split, &out4[0], &out4[1], &out4[2], &out4[3]);
 }
@@ -1050,10 +1052,7 @@ extern "C" int zse_gemm_w4_splits(int M, int N, int K, int k_split) {
   int sm_count = 148, dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
   if (sm_count <= 0) sm_count = 148;
-  if (!(g_w4_mode & 4)) {
-    const int gks = gemv_w4_plan(M, N, K, kEpiPartialF32, sm_count, k_split);
-    if (gks > 0) return gks;
-  }
+  if (takes_small(M, K, kEpiPartialF32, k_split)) return gemm_w4_small_planes(N, K, k_split);
   if (M > 64) return gemm_pair_planes(M, N, K, k_split);
   int R = 1, ks = 1, cluster = 1, dual = 0;
   plan_w4(M, N, K, kEpiPartialF32, sm_count, k_split, &R, &ks, &cluster, &dual);

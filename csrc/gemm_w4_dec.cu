@@ -1414,6 +1414,15 @@ static int run_dec(bool w8, const void* w_tiled, const void* x, int x_rows_cap, 
       (reinterpret_cast<uintptr_t>(bias) & 15))
     return ZSE_ERR_ALIGN;
   if (epilogue == kDecF32 ? (ldo % 4) : (ldo % 8)) return ZSE_ERR_ALIGN;
+  if (!w8 && epilogue != kDecAllReduceNorm && gemm_w4_small_takes(M, K)) {
+    const int epi = epilogue == kDecF16 ? kEpiF16 : epilogue == kDecSwiGLU ? kEpiSwiGLU
+                    : epilogue == kDecF32 ? kEpiPartialF32 : kEpiQkvRope;
+    SmallRope sr{};
+    if (rope != nullptr)
+      sr = SmallRope{rope->positions, rope->slots, rope->cos_sin, rope->kv_layer, rope->nh, rope->nkv, rope->block_size,
+                     rope->max_position};
+    return gemm_w4_small_run(w_tiled, x, bias, out, M, N, K, ldo, epi, 1, &sr, reinterpret_cast<cudaStream_t>(stream));
+  }
   const int sm_count = dec_sm_count();
   const int k_stages = K / kW4StageK;
   const int n_tiles = epilogue == kDecSwiGLU ? (N / 2 + 63) / 64 : (N + kTileN - 1) / kTileN;

@@ -47,9 +47,8 @@ KERNEL_TABLE: Dict[str, Tuple[str, str]] = {
                                              "64 tokens can take the persistent kernel gemm_w4_dec"),
     "tiled_dequant_matmul_int8": ("gemm_w8_dec", "tcgen05, the INT4 decode kernel's pipeline with 8-bit chunks: weights "
                                                  "stay INT8 in memory and are dequantised into TMEM; passes of more "
-                                                 "than 64 tokens expand the layer into a shared fp16 scratch with "
-                                                 "dequant_w8_tiled and run gemm_f16"),
-    "dequant_gemv_int4": ("gemm_w4", "M <= 2 takes the CUDA-core GEMV inside the same entry point"),
+                                                 "than 64 tokens take gemm_w8"),
+    "dequant_gemv_int4": ("gemm_w4", "M <= 8 streams the weights through registers (csrc/gemm_w4_small.cu) inside the same entry point"),
     "batched_dequant_gemv_int4": ("gemm_w4", "small batches take the narrow tensor-core tile"),
     "fused_gate_up_gemv_int4": ("gemm_w4", "epilogue 1: gate and up rows interleaved, activation applied in the epilogue"),
     "fp16_gemv": ("gemm_f16", ""),
