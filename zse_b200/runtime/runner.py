@@ -46,7 +46,7 @@ def _bucket(n: int, buckets: Sequence[int]) -> int:
 
 
 class ModelRunner:
-    DECODE_BUCKETS = (1, 2, 4, 8, 16, 32, 64, 128, 256)
+    DECODE_BUCKETS = (1, 2, 4, 8, 16, 32, 64, 96, 128, 160, 192, 256)
 
     def __init__(self, model: DecoderModel, cache: KVCacheManager, max_batch_seqs: int = 64,
                  max_tokens_per_pass: int = 2048, max_seq_len: Optional[int] = None, use_graphs: Optional[bool] = None,
