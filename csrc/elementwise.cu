@@ -35,6 +35,7 @@ __global__ void embedding_kernel(const __half* __restrict__ table, const int* __
 // sum and the normalisation, so the residual is read once and written once.
 constexpr int kNormThreads = 256;
 constexpr int kNormMaxVec = 8;      // float4 per thread -> H <= 8192
+constexpr int kNormManyRows = 592;  // rows from which add_rmsnorm_rows_kernel is the better one (four an SM)
 
 __device__ __forceinline__ float block_sum(float v, float* red) {
   v = warp_sum(v);
@@ -137,6 +138,74 @@ add_rmsnorm_kernel(float* __restrict__ residual, const float* __restrict__ parti
   }
 }
 
+// The same for passes of many rows: a row takes as few threads as hold it in registers (blockDim.x * 8 float4 >= H), so that an
+// SM works on many rows at once, and all loads of a plane are issued before the first addition.  8150 rows of 5120, one plane:
+// 213 us in a wide CTA a row, which waits for one row at a time; the floor is 91.
+__global__ void __launch_bounds__(kNormThreads)
+add_rmsnorm_rows_kernel(float* __restrict__ residual, const float* __restrict__ partials, int n_partials,
+                        const __half* __restrict__ add_f16, const __half* __restrict__ weight, __half* __restrict__ out,
+                        int M, int H, float eps) {
+  __shared__ float red[32];
+  pdl_launch_dependents();
+  pdl_wait();
+  const size_t base = size_t(blockIdx.x) * H, plane = size_t(M) * H;
+  const int nvec = H / 4;
+  float4 v[kNormMaxVec];
+#pragma unroll
+  for (int j = 0; j < kNormMaxVec; ++j) {
+    const int i = threadIdx.x + j * blockDim.x;
+    v[j] = residual != nullptr && i < nvec ? reinterpret_cast<const float4*>(residual + base)[i] : make_float4(0, 0, 0, 0);
+  }
+  for (int p = 0; p < n_partials; ++p) {
+    const float4* src = reinterpret_cast<const float4*>(partials + p * plane + base);
+    float4 y[kNormMaxVec];
+#pragma unroll
+    for (int j = 0; j < kNormMaxVec; ++j) {
+      const int i = threadIdx.x + j * blockDim.x;
+      y[j] = i < nvec ? __ldcs(src + i) : make_float4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int j = 0; j < kNormMaxVec; ++j) {
+      v[j].x += y[j].x; v[j].y += y[j].y; v[j].z += y[j].z; v[j].w += y[j].w;
+    }
+  }
+  if (add_f16 != nullptr) {
+#pragma unroll
+    for (int j = 0; j < kNormMaxVec; ++j) {
+      const int i = threadIdx.x + j * blockDim.x;
+      if (i < nvec) {
+        const uint2 raw = reinterpret_cast<const uint2*>(add_f16 + base)[i];
+        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
+        const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+        v[j].x += a.x; v[j].y += a.y; v[j].z += b.x; v[j].w += b.y;
+      }
+    }
+  }
+  float ss = 0.f;
+  const bool store = residual != nullptr && (n_partials > 0 || add_f16 != nullptr);
+#pragma unroll
+  for (int j = 0; j < kNormMaxVec; ++j) {
+    const int i = threadIdx.x + j * blockDim.x;
+    if (store && i < nvec) reinterpret_cast<float4*>(residual + base)[i] = v[j];
+    ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+  }
+  if (out == nullptr) return;
+  const float inv = rsqrtf(block_sum(ss, red) / float(H) + eps);
+#pragma unroll
+  for (int j = 0; j < kNormMaxVec; ++j) {
+    const int i = threadIdx.x + j * blockDim.x;
+    if (i < nvec) {
+      const uint2 wr = reinterpret_cast<const uint2*>(weight)[i];
+      const float2 w0 = __half22float2(*reinterpret_cast<const __half2*>(&wr.x));
+      const float2 w1 = __half22float2(*reinterpret_cast<const __half2*>(&wr.y));
+      uint2 pk;
+      pk.x = pack_half2(v[j].x * inv * w0.x, v[j].y * inv * w0.y);
+      pk.y = pack_half2(v[j].z * inv * w1.x, v[j].w * inv * w1.y);
+      reinterpret_cast<uint2*>(out + base)[i] = pk;
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_f16_kernel(const __half* __restrict__ x, const __half* __restrict__ weight, __half* __restrict__ out, int H,
                    float eps) {
@@ -232,8 +301,8 @@ __global__ void rope_kv_write_kernel(__half* __restrict__ qkv, __half* __restric
 
 // The same operation for the common case (q/k/v already fp16 in `qkv`, full rotary, head_dim a multiple of 16), built
 // for passes of many rows: ONE CTA per token instead of one per (token, head).  A thread owns eight rotation pairs
-// (i .. i+7 and their partners half a head away): it computes their sines and cosines once, then walks the heads
-// with two 16-byte loads and two 16-byte stores each.  The one-CTA-per-head form above spends 271 us on a prefill pass
+// (i .. i+7 and their partners half a head away): the CTA computes the token's sines and cosines once, then its threads walk
+// the heads with two 16-byte loads and two 16-byte stores each.  The one-CTA-per-head form above spends 271 us on a prefill pass
 // of 8 k tokens of the 14B shape (229 k CTAs of 64 threads, 2-byte accesses, a sincosf per element and head).
 __global__ void __launch_bounds__(256)
 rope_kv_write_vec_kernel(__half* __restrict__ qkv, __half* __restrict__ kv_layer, const int* __restrict__ positions,
@@ -247,9 +316,12 @@ rope_kv_write_vec_kernel(__half* __restrict__ qkv, __half* __restrict__ kv_layer
   const int half_rot = hd / 2, i0 = g * 8;
   const int heads = nh + 2 * nkv;
   const float pos = float(positions[t]);
+  __shared__ __align__(16) float sin_t[256], cos_t[256];         // of this token, computed once for all heads
+  for (int i = threadIdx.x; i < half_rot; i += blockDim.x) sincosf(pos * inv_freq[i], &sin_t[i], &cos_t[i]);
+  __syncthreads();
   float sn[8], cs[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) sincosf(pos * inv_freq[i0 + j], &sn[j], &cs[j]);
+  for (int j = 0; j < 8; ++j) sn[j] = sin_t[i0 + j], cs[j] = cos_t[i0 + j];
   const long long slot = slots[t];
   const long long blk = slot >= 0 ? slot / block_size : 0, off = slot >= 0 ? slot % block_size : 0;
   __half* row = qkv + size_t(t) * heads * hd;
@@ -280,6 +352,32 @@ rope_kv_write_vec_kernel(__half* __restrict__ qkv, __half* __restrict__ kv_layer
   }
 }
 
+__device__ __forceinline__ float gelu_tanh_f(float x) {
+  return 0.5f * x * (1.f + tanhf(0.7978845608f * (x + 0.044715f * x * x * x)));
+}
+
+// Eight outputs a thread with 16-byte accesses; grid (I / 8 / 256 rounded up, rows).  2670 rows of 14336: the pair-wise kernel
+// below takes 93 us, most of it 4-byte accesses and a 64-bit division per pair.
+__global__ void __launch_bounds__(256) swiglu_vec_kernel(const __half* __restrict__ gate_up, __half* __restrict__ out, int I,
+                                                         int gelu) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int j = (blockIdx.x * 256 + threadIdx.x) * 8;
+  if (j >= I) return;
+  const __half* row = gate_up + size_t(blockIdx.y) * 2 * I;
+  const uint4 g4 = __ldcs(reinterpret_cast<const uint4*>(row + j)), u4 = __ldcs(reinterpret_cast<const uint4*>(row + I + j));
+  const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w}, uw[4] = {u4.x, u4.y, u4.z, u4.w};
+  uint32_t o[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float2 g = __half22float2(*reinterpret_cast<const __half2*>(&gw[k]));
+    const float2 u = __half22float2(*reinterpret_cast<const __half2*>(&uw[k]));
+    o[k] = gelu ? pack_half2(clamp_f16(gelu_tanh_f(g.x) * u.x), clamp_f16(gelu_tanh_f(g.y) * u.y))
+                : pack_half2(clamp_f16(silu_f(g.x) * u.x), clamp_f16(silu_f(g.y) * u.y));
+  }
+  *reinterpret_cast<uint4*>(out + size_t(blockIdx.y) * I + j) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 __global__ void swiglu_kernel(const __half2* __restrict__ gate_up, __half2* __restrict__ out, int M, int I2,
                               int gelu) {
   // gate_up: [M, 2*I] as half2 -> rows of 2*I2 half2; out [M, I2]
@@ -290,8 +388,7 @@ __global__ void swiglu_kernel(const __half2* __restrict__ gate_up, __half2* __re
   const float2 u = __half22float2(gate_up[t * 2 * I2 + I2 + j]);
   float2 r;
   if (gelu) {
-    auto gl = [](float x) { return 0.5f * x * (1.f + tanhf(0.7978845608f * (x + 0.044715f * x * x * x))); };
-    r = make_float2(gl(g.x) * u.x, gl(g.y) * u.y);
+    r = make_float2(gelu_tanh_f(g.x) * u.x, gelu_tanh_f(g.y) * u.y);
   } else {
     r = make_float2(silu_f(g.x) * u.x, silu_f(g.y) * u.y);
   }
@@ -338,6 +435,14 @@ extern "C" int zse_add_rmsnorm(void* residual, const void* partials, int n_parti
                                const void* weight, void* out, int M, int H, float eps, void* stream) {
   if (M <= 0) return 0;
   if (H % 4 || H > 4 * kNormThreads * kNormMaxVec) return ZSE_ERR_SHAPE;
+  if (M >= kNormManyRows) {
+    const int threads = ((H / 4 + kNormMaxVec - 1) / kNormMaxVec + 31) / 32 * 32;
+    return launch_pdl(add_rmsnorm_rows_kernel, dim3(M), dim3(threads), 0, ST(stream), reinterpret_cast<float*>(residual),
+                      reinterpret_cast<const float*>(partials), n_partials, reinterpret_cast<const __half*>(add_f16),
+                      reinterpret_cast<const __half*>(weight), reinterpret_cast<__half*>(out), M, H, eps) == cudaSuccess
+               ? 0
+               : ZSE_ERR_LAUNCH;
+  }
   // CTAs per row: enough to put >= ~2 CTAs on every SM for small M, and few enough that H/4 splits evenly
   int cs = 1;
   while (cs < 8 && M * cs < 256 && (H / 4) % (cs * 2) == 0 && H / 4 / (cs * 2) >= 64) cs *= 2;
@@ -392,6 +497,11 @@ extern "C" int zse_rope_kv_write(void* qkv, void* kv_layer, const void* position
 extern "C" int zse_swiglu(const void* gate_up, void* out, int M, int I, int gelu, void* stream) {
   if (M <= 0) return 0;
   if (I % 2) return ZSE_ERR_SHAPE;
+  if (I % 8 == 0 && M <= 65535 && ((reinterpret_cast<uintptr_t>(gate_up) | reinterpret_cast<uintptr_t>(out)) & 15) == 0)
+    return launch_pdl(swiglu_vec_kernel, dim3((I / 8 + 255) / 256, M), dim3(256), 0, ST(stream),
+                      reinterpret_cast<const __half*>(gate_up), reinterpret_cast<__half*>(out), I, gelu) == cudaSuccess
+               ? 0
+               : ZSE_ERR_LAUNCH;
   const size_t total = size_t(M) * (I / 2);
   swiglu_kernel<<<unsigned((total + 255) / 256), 256, 0, ST(stream)>>>(reinterpret_cast<const __half2*>(gate_up),
                                                                        reinterpret_cast<__half2*>(out), M, I / 2, gelu);

@@ -93,6 +93,92 @@ headnorm_rope_kv_write_kernel(__half* __restrict__ qkv, int ld, __half* __restri
   }
 }
 
+// The same for passes of many rows: a CTA per token, a warp per head at a time.  Sines and cosines are computed once per token
+// instead of once per head, a lane takes four neighbouring pairs with 8-byte accesses (half a head a multiple of 4, <= 256).
+// 2670 tokens of 32 heads of 256: 85 thousand CTAs of one warp took 118 us.
+constexpr int kHeadNormManyRows = 296;     // two CTAs an SM; with fewer rows a warp per (token, head) spreads further
+
+__global__ void __launch_bounds__(256)
+headnorm_rope_rows_kernel(__half* __restrict__ qkv, int ld, __half* __restrict__ kv_layer, long long blk_stride,
+                          long long half_stride, const int* __restrict__ positions, const long long* __restrict__ slots,
+                          const float* __restrict__ freqs, const __half* __restrict__ q_norm_w,
+                          const __half* __restrict__ k_norm_w, int norm_v, int k_is_v, float eps, int nh, int nkv, int hd,
+                          int block_size) {
+  __shared__ float sin_t[256], cos_t[256];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.x, lane = threadIdx.x & 31, half = hd / 2;
+  const float pos = float(positions[t]);
+  for (int i = threadIdx.x; i < half; i += blockDim.x) {
+    const float f = freqs[i];
+    float s = 0.f, c = 1.f;                                    // frequency 0: the pair passes through
+    if (f != 0.f) sincosf(pos * f, &s, &c);
+    sin_t[i] = s, cos_t[i] = c;
+  }
+  __syncthreads();
+  const long long slot = slots[t];
+  const long long blk = slot >= 0 ? slot / block_size : 0, off = slot >= 0 ? slot % block_size : 0;
+  __half* row = qkv + size_t(t) * ld;
+  // a layer without v_proj has its v heads read the k projection, which the k heads leave as it is
+  for (int head = threadIdx.x >> 5; head < nh + 2 * nkv; head += blockDim.x >> 5) {
+    const bool is_q = head < nh, is_v = head >= nh + nkv;
+    const int kvh = is_q ? 0 : (is_v ? head - nh - nkv : head - nh);
+    const int col = is_q ? head * hd : (is_v && !k_is_v ? (nh + nkv + kvh) * hd : (nh + kvh) * hd);
+    const __half* w = is_q ? q_norm_w : (is_v ? nullptr : k_norm_w);
+    const bool normed = is_v ? norm_v != 0 : w != nullptr;
+    float a[2][4], b[2][4];
+    float ss = 0.f;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int i = lane * 4 + r * 128;
+      const bool in = i < half;
+      const uint2 va = in ? *reinterpret_cast<const uint2*>(row + col + i) : make_uint2(0, 0);
+      const uint2 vb = in ? *reinterpret_cast<const uint2*>(row + col + half + i) : make_uint2(0, 0);
+      const float2 a0 = __half22float2(*reinterpret_cast<const __half2*>(&va.x)),
+                   a1 = __half22float2(*reinterpret_cast<const __half2*>(&va.y)),
+                   b0 = __half22float2(*reinterpret_cast<const __half2*>(&vb.x)),
+                   b1 = __half22float2(*reinterpret_cast<const __half2*>(&vb.y));
+      a[r][0] = a0.x, a[r][1] = a0.y, a[r][2] = a1.x, a[r][3] = a1.y;
+      b[r][0] = b0.x, b[r][1] = b0.y, b[r][2] = b1.x, b[r][3] = b1.y;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) ss += a[r][k] * a[r][k] + b[r][k] * b[r][k];
+    }
+    float inv = 1.f;
+    if (normed) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      inv = rsqrtf(ss / float(hd) + eps);
+    }
+    __half* dst = nullptr;
+    if (is_q) dst = row + col;
+    else if (slot >= 0) dst = kv_layer + blk * blk_stride + (is_v ? half_stride : 0) + (size_t(kvh) * block_size + off) * hd;
+    if (dst == nullptr) continue;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int i = lane * 4 + r * 128;
+      if (i >= half) break;
+      float x[4], y[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        x[k] = a[r][k] * inv, y[k] = b[r][k] * inv;
+        if (normed && w != nullptr) {
+          x[k] *= __half2float(w[i + k]);
+          y[k] *= __half2float(w[i + half + k]);
+        }
+        if (!is_v) {
+          const float s = sin_t[i + k], c = cos_t[i + k];
+          const float rx = x[k] * c - y[k] * s, ry = y[k] * c + x[k] * s;
+          x[k] = rx, y[k] = ry;
+        }
+      }
+      *reinterpret_cast<uint2*>(dst + i) = make_uint2(pack_half2(clamp_f16(x[0]), clamp_f16(x[1])),
+                                                      pack_half2(clamp_f16(x[2]), clamp_f16(x[3])));
+      *reinterpret_cast<uint2*>(dst + half + i) = make_uint2(pack_half2(clamp_f16(y[0]), clamp_f16(y[1])),
+                                                             pack_half2(clamp_f16(y[2]), clamp_f16(y[3])));
+    }
+  }
+}
+
 // ---- generic paged attention ------------------------------------------------------------------------------------
 constexpr int kGenWarps = 8;
 
@@ -284,6 +370,71 @@ __device__ __forceinline__ float cta_sum(float v, float* red) {
   return total;
 }
 
+// Passes of many rows: as few threads a row as hold it in registers (blockDim.x * 8 vectors of four >= H), so that an SM works
+// on many rows at once, with 16-byte accesses to the residual.  2670 rows of 3584: 99 us with a wide CTA a row.
+constexpr int kPostNormVec = 8;
+constexpr int kPostNormManyRows = 592;
+
+__global__ void __launch_bounds__(256)
+norm_add_rmsnorm_rows_kernel(const __half* __restrict__ x, const __half* __restrict__ w_post, float* __restrict__ residual,
+                             const __half* __restrict__ scalar, const __half* __restrict__ w_next,
+                             __half* __restrict__ out, int H, float eps) {
+  __shared__ float red[32];
+  pdl_launch_dependents();
+  const float sc = scalar != nullptr ? __half2float(scalar[0]) : 1.f;
+  pdl_wait();
+  const size_t base = size_t(blockIdx.x) * H;
+  const int nvec = H / 4;
+  uint2 xr[kPostNormVec];
+  float4 rv[kPostNormVec];
+#pragma unroll
+  for (int k = 0; k < kPostNormVec; ++k) {
+    const int i = threadIdx.x + k * blockDim.x;
+    xr[k] = i < nvec ? reinterpret_cast<const uint2*>(x + base)[i] : make_uint2(0, 0);
+    rv[k] = i < nvec ? reinterpret_cast<const float4*>(residual + base)[i] : make_float4(0, 0, 0, 0);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < kPostNormVec; ++k) {
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&xr[k].x)),
+                 b = __half22float2(*reinterpret_cast<const __half2*>(&xr[k].y));
+    ss += a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y;
+  }
+  const float inv = rsqrtf(cta_sum(ss, red) / float(H) + eps);
+  float ss2 = 0.f;
+#pragma unroll
+  for (int k = 0; k < kPostNormVec; ++k) {
+    const int i = threadIdx.x + k * blockDim.x;
+    if (i < nvec) {
+      const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&xr[k].x)),
+                   b = __half22float2(*reinterpret_cast<const __half2*>(&xr[k].y));
+      const uint2 wr = reinterpret_cast<const uint2*>(w_post)[i];
+      const float2 w0 = __half22float2(*reinterpret_cast<const __half2*>(&wr.x)),
+                   w1 = __half22float2(*reinterpret_cast<const __half2*>(&wr.y));
+      rv[k].x = (rv[k].x + a.x * inv * w0.x) * sc;
+      rv[k].y = (rv[k].y + a.y * inv * w0.y) * sc;
+      rv[k].z = (rv[k].z + b.x * inv * w1.x) * sc;
+      rv[k].w = (rv[k].w + b.y * inv * w1.y) * sc;
+      reinterpret_cast<float4*>(residual + base)[i] = rv[k];
+      ss2 += rv[k].x * rv[k].x + rv[k].y * rv[k].y + rv[k].z * rv[k].z + rv[k].w * rv[k].w;
+    }
+  }
+  if (out == nullptr) return;
+  const float inv2 = rsqrtf(cta_sum(ss2, red) / float(H) + eps);
+#pragma unroll
+  for (int k = 0; k < kPostNormVec; ++k) {
+    const int i = threadIdx.x + k * blockDim.x;
+    if (i < nvec) {
+      const uint2 wr = reinterpret_cast<const uint2*>(w_next)[i];
+      const float2 w0 = __half22float2(*reinterpret_cast<const __half2*>(&wr.x)),
+                   w1 = __half22float2(*reinterpret_cast<const __half2*>(&wr.y));
+      reinterpret_cast<uint2*>(out + base)[i] =
+          make_uint2(pack_half2(clamp_f16(rv[k].x * inv2 * w0.x), clamp_f16(rv[k].y * inv2 * w0.y)),
+                     pack_half2(clamp_f16(rv[k].z * inv2 * w1.x), clamp_f16(rv[k].w * inv2 * w1.y)));
+    }
+  }
+}
+
 // One CTA per row.  Rows of up to kPostNormThreads * kPostNormRegs elements are held in registers (one read of x and
 // of the residual, all loads issued before the first reduction); longer rows take the looping version.
 constexpr int kPostNormRegs = 32;
@@ -372,6 +523,15 @@ extern "C" int zse_headnorm_rope_kv_write(void* qkv, int ld, void* kv_layer, int
                                           float eps, int M, int nh, int nkv, int hd, int block_size, void* stream) {
   if (M <= 0) return 0;
   if (hd % 2 || hd > 64 * kGemmaMaxPairsPerLane || nh <= 0 || nkv <= 0) return ZSE_ERR_SHAPE;
+  if (M >= kHeadNormManyRows && hd % 8 == 0 && ld % 4 == 0 && (blk_stride & 3) == 0 && (half_stride & 3) == 0 &&
+      ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(kv_layer)) & 7) == 0)
+    return launch_pdl(headnorm_rope_rows_kernel, dim3(M), dim3(256), 0, ST(stream), reinterpret_cast<__half*>(qkv), ld,
+                      reinterpret_cast<__half*>(kv_layer), (long long)blk_stride, (long long)half_stride,
+                      reinterpret_cast<const int*>(positions), reinterpret_cast<const long long*>(slots),
+                      reinterpret_cast<const float*>(freqs), reinterpret_cast<const __half*>(q_norm_w),
+                      reinterpret_cast<const __half*>(k_norm_w), norm_v, k_is_v, eps, nh, nkv, hd, block_size) == cudaSuccess
+               ? 0
+               : ZSE_ERR_LAUNCH;
   dim3 grid(M, nh + 2 * nkv);
   return launch_pdl(headnorm_rope_kv_write_kernel, grid, dim3(32), 0, ST(stream), reinterpret_cast<__half*>(qkv), ld,
                     reinterpret_cast<__half*>(kv_layer), (long long)blk_stride, (long long)half_stride,
@@ -435,6 +595,16 @@ extern "C" int zse_norm_add_rmsnorm(const void* x, const void* w_post, void* res
                                     const void* w_next, void* out, int M, int H, float eps, void* stream) {
   if (M <= 0) return 0;
   if (H <= 0 || (out != nullptr && w_next == nullptr)) return ZSE_ERR_SHAPE;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w_post) | reinterpret_cast<uintptr_t>(w_next) |
+                       reinterpret_cast<uintptr_t>(out);
+  if (M >= kPostNormManyRows && H % 4 == 0 && H <= 4 * 256 * kPostNormVec && (at & 7) == 0 &&
+      (reinterpret_cast<uintptr_t>(residual) & 15) == 0) {
+    const int threads = ((H / 4 + kPostNormVec - 1) / kPostNormVec + 31) / 32 * 32;
+    return launch_pdl(norm_add_rmsnorm_rows_kernel, dim3(M), dim3(threads), 0, ST(stream), reinterpret_cast<const __half*>(x),
+                      reinterpret_cast<const __half*>(w_post), reinterpret_cast<float*>(residual),
+                      reinterpret_cast<const __half*>(scalar), reinterpret_cast<const __half*>(w_next),
+                      reinterpret_cast<__half*>(out), H, eps) == cudaSuccess ? 0 : ZSE_ERR_LAUNCH;
+  }
   auto kern = H <= kPostNormThreads * kPostNormRegs ? norm_add_rmsnorm_kernel<true> : norm_add_rmsnorm_kernel<false>;
   return launch_pdl(kern, dim3(M), dim3(kPostNormThreads), 0, ST(stream), reinterpret_cast<const __half*>(x),
                     reinterpret_cast<const __half*>(w_post), reinterpret_cast<float*>(residual),
