@@ -235,7 +235,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     }
   } else if (warp == 5) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    {                                                  // all lanes walk, one issues (see elect_one)
+      auto all = [](bool v) { return __all_sync(0xffffffffu, v) != 0; };
       constexpr uint32_t idesc_qk = make_idesc_f16(kTcRows, kTcKv);
       constexpr uint32_t idesc_pv = make_idesc_f16(kTcRows, kTcHd) | (1u << 16);       // B is MN-major
       const uint64_t q_desc = make_desc_sw128(smem_u32(q_s));
@@ -243,35 +244,41 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
       // V [keys][head_dim] as the MN-major B operand: 64 head_dim elements per 128-byte row, eight keys per 1024 bytes,
       // the second half of head_dim 16 KB further on
       const uint32_t mn64 = uint32_t(kTcTileBytes / 2), k8 = 1024u;
-      bool ok = mbar_wait_spin(&bars->q_full, 0, abort_flag, a.status, 43, 0);
+      const bool ok = all(mbar_wait_spin(&bars->q_full, 0, abort_flag, a.status, 43, 0));
       uint32_t ph = 0;
       for (int t = 0; t < n_tiles && ok; ++t) {
-        if (!mbar_wait_spin(&bars->k_full, ph, abort_flag, a.status, 44, t)) break;
-        ATIME(t, 0);
+        if (!all(mbar_wait_spin(&bars->k_full, ph, abort_flag, a.status, 44, t))) break;
+        if (lane == 0) ATIME(t, 0);
         // the probabilities of the previous tile live in the columns this product overwrites: let P V finish reading
         // them first (v_empty of tile t-1 is committed behind that product)
-        if (t > 0 && !mbar_wait_spin(&bars->v_empty, ph ^ 1, abort_flag, a.status, 49, t)) break;
-        ATIME(t, 1);
+        if (t > 0 && !all(mbar_wait_spin(&bars->v_empty, ph ^ 1, abort_flag, a.status, 49, t))) break;
+        if (lane == 0) ATIME(t, 1);
         tc_fence_after_sync();
+        if (elect_one()) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const uint64_t adv = uint64_t((j >> 2) * (kTcTileBytes / 2 >> 4) + (j & 3) * 2);
-          umma_ss(tm_s, q_desc + adv, k_desc + adv, idesc_qk, j != 0);
+          for (int j = 0; j < 8; ++j) {
+            const uint64_t adv = uint64_t((j >> 2) * (kTcTileBytes / 2 >> 4) + (j & 3) * 2);
+            umma_ss(tm_s, q_desc + adv, k_desc + adv, idesc_qk, j != 0);
+          }
+          tc_commit(&bars->s_full);                   // S complete (and every earlier MMA, i.e. the previous P V)
         }
-        tc_commit(&bars->s_full);                     // S complete (and every earlier MMA, i.e. the previous P V)
-        ATIME(t, 2);
-        if (!mbar_wait_spin(&bars->v_full, ph, abort_flag, a.status, 45, t)) break;
-        ATIME(t, 3);
-        if (!mbar_wait_spin(&bars->p_full, ph, abort_flag, a.status, 46, t)) break;
-        ATIME(t, 4);
+        __syncwarp();
+        if (lane == 0) ATIME(t, 2);
+        if (!all(mbar_wait_spin(&bars->v_full, ph, abort_flag, a.status, 45, t))) break;
+        if (lane == 0) ATIME(t, 3);
+        if (!all(mbar_wait_spin(&bars->p_full, ph, abort_flag, a.status, 46, t))) break;
+        if (lane == 0) ATIME(t, 4);
         tc_fence_after_sync();
+        if (elect_one()) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {                 // 16 keys per step: two groups of eight cache rows
-          const uint64_t v_desc = make_desc_sw128_mn(smem_u32(v_s) + j * 2048, mn64, k8);
-          umma_ts(tm_o, tm_p + j * 8, v_desc, idesc_pv, (t != 0) || (j != 0));
+          for (int j = 0; j < 8; ++j) {               // 16 keys per step: two groups of eight cache rows
+            const uint64_t v_desc = make_desc_sw128_mn(smem_u32(v_s) + j * 2048, mn64, k8);
+            umma_ts(tm_o, tm_p + j * 8, v_desc, idesc_pv, (t != 0) || (j != 0));
+          }
+          tc_commit(&bars->v_empty);
         }
-        tc_commit(&bars->v_empty);
-        ATIME(t, 5);
+        __syncwarp();
+        if (lane == 0) ATIME(t, 5);
         ph ^= 1;
       }
     }
