@@ -4,12 +4,11 @@
 // 16-token tile of one kv head is a contiguous hd*32-byte run.  Block id -1 in a block table is a hole left by
 // eviction and is skipped, as in the reference (zse-engine/zse_engine/orchestrator/kernels.py:571,653).
 //
-// attn_decode_kernel  - one query token per sequence.  A CTA owns (kv head, sequence, split): all G = nh/nkv query
-//                       heads of the kv head form the 16-row M dimension of m16n8k16 MMAs, so K and V are read once
-//                       per kv head (the reference reads them once per query head, kernels.py:524-671).  Each warp
-//                       streams its own 16-token tiles through a private 3-stage cp.async ring (no CTA barriers in
-//                       the main loop), keeps an online-softmax state in registers, and the four warps merge at the
-//                       end.  With num_splits > 1 the CTA writes (O, m, l) to scratch and attn_combine_kernel merges.
+// attn_decode_kernel  - one query token per sequence.  K and V are read once per kv head for all G = nh/nkv query heads (the
+//                       reference reads them once per query head, kernels.py:524-671).  One grid of as many CTAs as fit; each
+//                       takes an equal run of 16-token tiles over all sequences and kv heads, its four warps
+//                       stream tiles through private 3-stage cp.async rings that run on from one item into the next (no CTA
+//                       barriers in the main loop), keep an online softmax in registers and merge at the end of an item.
 // attn_prefill_kernel - causal attention of a chunk of query tokens against everything already in the cache
 //                       (earlier chunks included), flash-attention style: 64 query rows per CTA, 64-token KV tiles,
 //                       online softmax.  Serves prefill, chunked prefill and speculative verification
@@ -49,7 +48,6 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
 }
 
 constexpr int kDecWarps = 4;
-constexpr int kDecStages = 3;
 constexpr float kLog2e = 1.4426950408889634f;
 
 // Shared-memory tile: `rows` rows of HD halfs; 16-byte chunk c of row r lives at chunk (c ^ (r & 7)).
@@ -58,233 +56,402 @@ __device__ __forceinline__ uint32_t tile_off(int row, int chunk) {
   return uint32_t(row * (HD * 2) + ((chunk ^ (row & 7)) << 4));
 }
 
+// ---- decode: how the work is cut -------------------------------------------------------------------------------------------
+// All 16-token tiles of all (sequence, kv head) items stand in one line, sequence by sequence.  With num_splits > 1 every CTA
+// takes the same number of them, `per`, whatever items they belong to; an item that lies in several CTAs is merged from scratch
+// by attn_combine_kernel (at most num_splits - 1 pieces: `per` is raised for that if one sequence is very long).  The last of a
+// head's num_splits records in scratch says how many pieces there are.  With num_splits < 3 items stay whole.
+template <int HD, int NB>
+constexpr int kDecodeStages = HD == 256 && NB == 2 ? 2 : 3;       // of a warp's ring
+__device__ __forceinline__ int seq_tiles(int len, int window) {
+  return ((len + 15) >> 4) - ((window > 0 ? max(0, len - window) : 0) >> 4);
+}
+__device__ __forceinline__ int tiles_per_cta(int total, int longest, int ctas, int num_splits) {
+  return max(kDecWarps, max((total + ctas - 1) / ctas, (longest + num_splits - 3) / (num_splits - 2)));
+}
+__device__ __forceinline__ int* piece_count(float* scratch, int row, int num_splits, int hd) {
+  return reinterpret_cast<int*>(scratch + (size_t(row + 1) * num_splits - 1) * (hd + 2));
+}
+// 2^x in one instruction: scores below the maximum, so the range handling of exp2f() is not needed
+__device__ __forceinline__ float ex2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
+  uint32_t y;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+  return y;
+}
+
 // EXT adds what the Gemma family needs: scores soft-capped as cap*tanh(s/cap) and a sliding window (only the last
 // `window` tokens are seen).  The cache is addressed through strides (block, K->V), so a layer may be a view into a
-// pool with wider rows.
-template <int HD, bool EXT>
+// pool with wider rows.  NB: blocks of eight query heads per kv head.
+//
+// Tokens are the 16 rows of the products and query heads their 8 columns (S^T = K Q^T, O^T = V^T P^T; the probabilities change
+// sides with movmatrix).  With heads as the rows, half of every product, every exponential and half of the accumulators were for
+// heads that do not exist (groups of 2 to 8): 385 instructions a tile and 164 registers.
+template <int HD, bool EXT, int NB>
 __global__ void __launch_bounds__(kDecWarps * 32)
 attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restrict__ kv, const int* __restrict__ bt,
                    int max_blocks, const int* __restrict__ seq_lens, __half* __restrict__ out, int ldo,
-                   float* __restrict__ scratch, int nh, int nkv, int block_size, int num_splits, float scale_log2,
-                   long long blk_stride, long long half_stride, float softcap, int window) {
+                   float* __restrict__ scratch, int num_seqs, int nh, int nkv, int block_size, int block_shift,
+                   int num_splits, float scale_log2, long long blk_stride, long long half_stride, float softcap, int window) {
   constexpr int kTileBytes = 16 * HD * 2;              // one 16-token K (or V) tile
+  constexpr int kDecStages = kDecodeStages<HD, NB>;
   constexpr int kChunksPerRow = HD / 8;
-  constexpr int kKSteps = HD / 16;
-  constexpr int kNTilesO = HD / 8;
+  constexpr int kSteps = HD / 16;
+  constexpr int kHeads = 8 * NB;
+  constexpr int kPitch = HD + 4;                       // floats per head in the merge buffers: conflict-free
+  constexpr int kBuf = kHeads * kPitch + 2 * kHeads;   // O, then m and l per head
   extern __shared__ __align__(128) uint8_t smem[];
+  float* merge = reinterpret_cast<float*>(smem + kDecWarps * kDecStages * 2 * kTileBytes);
+  int* prefix = reinterpret_cast<int*>(merge + 3 * kBuf);      // [num_seqs + 1] tiles x nkv before a sequence
+  __shared__ int s_longest;
   pdl_launch_dependents();
   pdl_wait();
-  const int kvh = blockIdx.x, seq = blockIdx.y, split = blockIdx.z;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t2 = (lane & 3) * 2;
   const int G = nh / nkv;
-  const int len = seq_lens[seq];
-  const int first_tok = (EXT && window > 0) ? max(0, len - window) : 0;
-  const int total_tiles = (len + 15) >> 4;
-  const int tile0 = first_tok >> 4;
-  const int per_split = (total_tiles - tile0 + num_splits - 1) / num_splits;
-  const int tile_begin = tile0 + split * per_split;
-  const int tile_end = min(total_tiles, tile_begin + per_split);
-  const int my_count = tile_end > tile_begin + warp ? (tile_end - tile_begin - warp + kDecWarps - 1) / kDecWarps : 0;
-
-  uint8_t* ring = smem + warp * (kDecStages * 2 * kTileBytes);
-  const int* my_bt = bt + size_t(seq) * max_blocks;
-  const size_t kv_head_stride = size_t(block_size) * HD;        // elements between kv heads inside a block half
-
-  // Q fragments: rows = query heads of this kv head (zero beyond G)
-  uint32_t qa[kKSteps][4];
-  {
-    const int g0 = lane >> 2, g1 = g0 + 8, c = (lane & 3) * 2;
-    const __half* q0 = q + size_t(seq) * ldq + size_t(kvh * G + g0) * HD;
-    const __half* q1 = q + size_t(seq) * ldq + size_t(kvh * G + g1) * HD;
+  // ---- lengths -> prefix sums of the tiles.  Up to 32 sequences stay in a warp's lanes (no barrier before the first load of
+  // keys); more go through shared memory.
+  const bool in_lanes = num_seqs <= 32;
+  int my_n = 0, my_incl = 0, longest = 0, total = 0;
+  if (in_lanes) {
+    my_n = lane < num_seqs ? seq_tiles(seq_lens[lane], EXT ? window : 0) : 0;
+    my_incl = my_n * nkv;
 #pragma unroll
-    for (int kk = 0; kk < kKSteps; ++kk) {
-      qa[kk][0] = g0 < G ? *reinterpret_cast<const uint32_t*>(q0 + kk * 16 + c) : 0u;
-      qa[kk][1] = g1 < G ? *reinterpret_cast<const uint32_t*>(q1 + kk * 16 + c) : 0u;
-      qa[kk][2] = g0 < G ? *reinterpret_cast<const uint32_t*>(q0 + kk * 16 + 8 + c) : 0u;
-      qa[kk][3] = g1 < G ? *reinterpret_cast<const uint32_t*>(q1 + kk * 16 + 8 + c) : 0u;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, my_incl, o);
+      if (lane >= o) my_incl += u;
     }
+    longest = __reduce_max_sync(0xffffffffu, my_n);
+    total = __shfl_sync(0xffffffffu, my_incl, 31);
+  } else {
+    if (threadIdx.x == 0) s_longest = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < num_seqs; i += blockDim.x) {
+      const int n = seq_tiles(seq_lens[i], EXT ? window : 0);
+      prefix[i + 1] = n * nkv;
+      atomicMax(&s_longest, n);
+    }
+    __syncthreads();
+    if (warp == 0) {
+      int carry = 0;
+      for (int i = 0; i < num_seqs; i += 32) {
+        int v = i + lane < num_seqs ? prefix[i + lane + 1] : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, v, o);
+          if (lane >= o) v += u;
+        }
+        if (i + lane < num_seqs) prefix[i + lane + 1] = carry + v;
+        carry += __shfl_sync(0xffffffffu, v, 31);
+      }
+      if (lane == 0) prefix[0] = 0;
+    }
+    __syncthreads();
+    longest = s_longest;
+    total = prefix[num_seqs];
   }
+  auto tiles_of = [&](int i) {
+    return in_lanes ? __shfl_sync(0xffffffffu, my_n, i) : (prefix[i + 1] - prefix[i]) / nkv;
+  };
+  const bool whole = num_splits < 3;                   // items are not cut: CTA i has item i
+  const int per = whole ? 1 : tiles_per_cta(total, longest, gridDim.x, num_splits);
+  const int p_begin = whole ? int(blockIdx.x) : min(total, int(blockIdx.x) * per);
+  const int p_end = whole ? int(blockIdx.x) + 1 : min(total, p_begin + per);
 
-  auto issue = [&](int i) {       // i-th tile of this warp -> ring slot i % stages; always commits a group
-    if (i < my_count) {
-      const int tile = tile_begin + warp + i * kDecWarps;
-      const int tok = tile << 4;
-      const int blk = my_bt[tok / block_size];
+  struct Seg {
+    int seq, kvh, first, n, tiles;                     // tiles first .. first + n - 1 of `tiles` of the item
+  };
+  // the segment at position p (p < p_end), and the position behind it; the whole warp calls it
+  auto segment = [&](int p, Seg& sg) {
+    if (whole) {
+      sg.seq = unsigned(p) / unsigned(nkv), sg.kvh = p - sg.seq * nkv;
+      sg.first = 0;
+      sg.tiles = sg.n = tiles_of(sg.seq);
+      return p + 1;
+    }
+    int begin;
+    if (in_lanes) {
+      sg.seq = __popc(__ballot_sync(0xffffffffu, my_incl <= p));
+      sg.tiles = __shfl_sync(0xffffffffu, my_n, sg.seq);
+      begin = __shfl_sync(0xffffffffu, my_incl, sg.seq) - sg.tiles * nkv;
+    } else {
+      int lo = 0, hi = num_seqs;
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (prefix[mid] <= p) lo = mid; else hi = mid;
+      }
+      sg.seq = lo;
+      sg.tiles = unsigned(prefix[lo + 1] - prefix[lo]) / unsigned(nkv);
+      begin = prefix[lo];
+    }
+    sg.kvh = unsigned(p - begin) / unsigned(sg.tiles);
+    sg.first = p - begin - sg.kvh * sg.tiles;
+    sg.n = min(sg.tiles - sg.first, p_end - p);
+    return p + sg.n;
+  };
+
+  // ---- this warp's tiles, one after the other over all segments: what is fetched next
+  uint8_t* ring = smem + warp * (kDecStages * 2 * kTileBytes);
+  Seg fs{};
+  int fp = p_begin, fi = 0, f_tile0 = 0;
+  bool f_live = true;
+  fs.n = 0;
+  auto f_seek = [&]() {                                // fi past the end of the segment: on to one with a tile for this warp
+    while (fi >= fs.n) {
+      if (fp >= p_end) {
+        f_live = false;
+        return;
+      }
+      fp = segment(fp, fs);
+      fi = warp;
+      f_tile0 = (EXT && window > 0 ? max(0, seq_lens[fs.seq] - window) >> 4 : 0) + fs.first;
+    }
+  };
+  f_seek();
+  uint32_t holes = 0;                                  // bit = ring slot whose tile lies in a dropped block
+  auto issue = [&](int slot) {                         // next tile -> ring slot; always commits a group
+    holes &= ~(1u << slot);
+    if (f_live) {
+      const int tile = f_tile0 + fi;
+      const int bi = block_shift >= 0 ? tile >> block_shift : tile / (block_size >> 4);
+      const int in = tile - bi * (block_size >> 4);
+      const int blk = bt[size_t(fs.seq) * max_blocks + bi];
       if (blk >= 0) {
-        const __half* ksrc = kv + size_t(blk) * blk_stride + size_t(kvh) * kv_head_stride + size_t(tok % block_size) * HD;
+        const __half* ksrc = kv + size_t(blk) * blk_stride + (size_t(fs.kvh) * block_size + in * 16) * HD + lane * 8;
         const __half* vsrc = ksrc + half_stride;
-        uint8_t* kd = ring + (i % kDecStages) * 2 * kTileBytes;
-        uint8_t* vd = kd + kTileBytes;
+        uint8_t* kd = ring + slot * 2 * kTileBytes;
 #pragma unroll
         for (int j = 0; j < kTileBytes / 512; ++j) {
           const int idx = j * 32 + lane;
-          const int row = idx / kChunksPerRow, ch = idx % kChunksPerRow;
-          cp_async16(kd + tile_off<HD>(row, ch), ksrc + idx * 8);
-          cp_async16(vd + tile_off<HD>(row, ch), vsrc + idx * 8);
+          const uint32_t off = tile_off<HD>(idx / kChunksPerRow, idx % kChunksPerRow);
+          cp_async16(kd + off, ksrc + j * 256);
+          cp_async16(kd + kTileBytes + off, vsrc + j * 256);
         }
+      } else {
+        holes |= 1u << slot;
       }
+      fi += kDecWarps;
+      f_seek();
     }
     cp_async_commit();
   };
-
-  float o[kNTilesO][4];
-#pragma unroll
-  for (int n = 0; n < kNTilesO; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
-
 #pragma unroll
   for (int i = 0; i < kDecStages - 1; ++i) issue(i);
 
-  for (int i = 0; i < my_count; ++i) {
-    cp_async_wait<kDecStages - 2>();
-    __syncwarp();
-    issue(i + kDecStages - 1);
-    const int tile = tile_begin + warp + i * kDecWarps;
-    const int tok = tile << 4;
-    if (my_bt[tok / block_size] < 0) continue;          // hole
-    const uint32_t kbase = smem_u32(ring + (i % kDecStages) * 2 * kTileBytes);
-    const uint32_t vbase = kbase + kTileBytes;
-
-    float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-    {
-      const int m = lane >> 3, rr = lane & 7;
-      const int row = (m >> 1) * 8 + rr;
+  for (int i = blockIdx.x; i < num_seqs; i += gridDim.x)       // sequences of nothing: zeros
+    if (tiles_of(i) == 0) {
+      for (int d = threadIdx.x; d < nh * HD; d += blockDim.x) out[size_t(i) * ldo + d] = __float2half_rn(0.f);
+      if (!whole)
+        for (int h = threadIdx.x; h < nh; h += blockDim.x) *piece_count(scratch, i * nh + h, num_splits, HD) = 1;
+    }
+  int slot = 0;
+  for (int p = p_begin; p < p_end;) {
+    Seg sg;
+    const int here = p;
+    p = segment(p, sg);
+    if (sg.n == 0) continue;                           // (a whole item: an empty sequence)
+    const int len = seq_lens[sg.seq];
+    const int first_tok = EXT && window > 0 ? max(0, len - window) : 0;
+    uint32_t qb[NB][kSteps][2];
 #pragma unroll
-      for (int kk = 0; kk < kKSteps; ++kk) {
-        uint32_t b0, b1, b2, b3;
-        ldsm_x4(kbase + tile_off<HD>(row, kk * 2 + (m & 1)), b0, b1, b2, b3);
-        mma16816(s[0], qa[kk], b0, b1);
-        mma16816(s[1], qa[kk], b2, b3);
+    for (int nb = 0; nb < NB; ++nb) {
+      const int h = nb * 8 + g;
+      const __half* src = q + size_t(sg.seq) * ldq + size_t(sg.kvh * G + h) * HD + t2;
+#pragma unroll
+      for (int kk = 0; kk < kSteps; ++kk) {
+        qb[nb][kk][0] = h < G ? *reinterpret_cast<const uint32_t*>(src + kk * 16) : 0u;
+        qb[nb][kk][1] = h < G ? *reinterpret_cast<const uint32_t*>(src + kk * 16 + 8) : 0u;
       }
     }
-    // scale, mask the tail, online softmax (rows lane/4 and lane/4 + 8)
-    float mx0 = -INFINITY, mx1 = -INFINITY;
+    float o[NB][kSteps][4], m[NB][2], l[NB][2];
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
+    for (int nb = 0; nb < NB; ++nb) {
+      m[nb][0] = m[nb][1] = -INFINITY;
+      l[nb][0] = l[nb][1] = 0.f;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int t = tok + j * 8 + (lane & 3) * 2 + (e & 1);
-        float v = s[j][e] * scale_log2;
-        if constexpr (EXT) {
-          if (softcap > 0.f) v = softcap * kLog2e * tanhf(v * (1.f / (kLog2e * softcap)));
-          if (t < first_tok) v = -INFINITY;
+      for (int d = 0; d < kSteps; ++d) o[nb][d][0] = o[nb][d][1] = o[nb][d][2] = o[nb][d][3] = 0.f;
+    }
+    for (int i = warp; i < sg.n; i += kDecWarps) {
+      cp_async_wait<kDecStages - 2>();
+      __syncwarp();
+      const bool hole = (holes >> slot) & 1u;
+      issue(slot == 0 ? kDecStages - 1 : slot - 1);    // the slot of the tile before this one
+      const uint32_t kbase = smem_u32(ring + slot * 2 * kTileBytes), vbase = kbase + kTileBytes;
+      slot = slot + 1 == kDecStages ? 0 : slot + 1;
+      if (hole) continue;
+      const int tok = ((first_tok >> 4) + sg.first + i) << 4;
+      const int mm = lane >> 3, rr = lane & 7;
+      float s[NB][2][4];                               // even and odd K steps apart: two chains
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[nb][0][e] = s[nb][1][e] = 0.f;
+#pragma unroll
+      for (int kk = 0; kk < kSteps; ++kk) {
+        uint32_t a[4];
+        ldsm_x4(kbase + tile_off<HD>((mm & 1) * 8 + rr, kk * 2 + (mm >> 1)), a[0], a[1], a[2], a[3]);
+#pragma unroll
+        for (int nb = 0; nb < NB; ++nb) mma16816(s[nb][kk & 1], a, qb[nb][kk][0], qb[nb][kk][1]);
+      }
+      const bool dead0 = tok + g >= len || (EXT && tok + g < first_tok);
+      const bool dead1 = tok + g + 8 >= len || (EXT && tok + g + 8 < first_tok);
+      uint32_t pb[NB][2];
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb) {
+        float v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          v[e] = (s[nb][0][e] + s[nb][1][e]) * scale_log2;
+          if constexpr (EXT) {
+            if (softcap > 0.f) v[e] = softcap * kLog2e * tanhf(v[e] * (1.f / (kLog2e * softcap)));
+          }
+          if (e < 2 ? dead0 : dead1) v[e] = -INFINITY;
         }
-        if (t >= len) v = -INFINITY;
-        s[j][e] = v;
-        if (e < 2) mx0 = fmaxf(mx0, v); else mx1 = fmaxf(mx1, v);
-      }
-    }
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-    const float n0 = fmaxf(m0, mx0), n1 = fmaxf(m1, mx1);
-    if (__any_sync(0xffffffffu, n0 > m0 || n1 > m1)) {
-      const float a0 = m0 == -INFINITY ? 0.f : exp2f(m0 - n0), a1 = m1 == -INFINITY ? 0.f : exp2f(m1 - n1);
-      l0 *= a0;
-      l1 *= a1;
+        float x0 = fmaxf(v[0], v[2]), x1 = fmaxf(v[1], v[3]);       // heads t2, t2 + 1
 #pragma unroll
-      for (int n = 0; n < kNTilesO; ++n) {
-        o[n][0] *= a0; o[n][1] *= a0; o[n][2] *= a1; o[n][3] *= a1;
-      }
-      m0 = n0;
-      m1 = n1;
-    }
-    uint32_t pa[4];
-    {
-      const float b0f = m0 == -INFINITY ? 0.f : m0, b1f = m1 == -INFINITY ? 0.f : m1;   // fully masked rows
-      const float p00 = exp2f(s[0][0] - b0f), p01 = exp2f(s[0][1] - b0f), p02 = exp2f(s[0][2] - b1f),
-                  p03 = exp2f(s[0][3] - b1f);
-      const float p10 = exp2f(s[1][0] - b0f), p11 = exp2f(s[1][1] - b0f), p12 = exp2f(s[1][2] - b1f),
-                  p13 = exp2f(s[1][3] - b1f);
-      l0 += p00 + p01 + p10 + p11;
-      l1 += p02 + p03 + p12 + p13;
-      pa[0] = pack_h2(p00, p01);
-      pa[1] = pack_h2(p02, p03);
-      pa[2] = pack_h2(p10, p11);
-      pa[3] = pack_h2(p12, p13);
-    }
-    {
-      const int m = lane >> 3, rr = lane & 7;
-      const int row = (m & 1) * 8 + rr;
+        for (int sh = 4; sh < 32; sh <<= 1) {
+          x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, sh));
+          x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, sh));
+        }
+        const float n0 = fmaxf(m[nb][0], x0), n1 = fmaxf(m[nb][1], x1);
+        if (__any_sync(0xffffffffu, n0 > m[nb][0] || n1 > m[nb][1])) {
+          const float a0 = m[nb][0] == -INFINITY ? 0.f : ex2_approx(m[nb][0] - n0);
+          const float a1 = m[nb][1] == -INFINITY ? 0.f : ex2_approx(m[nb][1] - n1);
+          l[nb][0] *= a0;
+          l[nb][1] *= a1;
 #pragma unroll
-      for (int p = 0; p < kNTilesO / 2; ++p) {
-        uint32_t b0, b1, b2, b3;
-        ldsm_x4_t(vbase + tile_off<HD>(row, p * 2 + (m >> 1)), b0, b1, b2, b3);
-        mma16816(o[2 * p], pa, b0, b1);
-        mma16816(o[2 * p + 1], pa, b2, b3);
+          for (int d = 0; d < kSteps; ++d) {
+            o[nb][d][0] *= a0; o[nb][d][1] *= a1; o[nb][d][2] *= a0; o[nb][d][3] *= a1;
+          }
+          m[nb][0] = n0;
+          m[nb][1] = n1;
+        }
+        const float b0 = m[nb][0] == -INFINITY ? 0.f : m[nb][0], b1 = m[nb][1] == -INFINITY ? 0.f : m[nb][1];
+        const float p00 = ex2_approx(v[0] - b0), p01 = ex2_approx(v[1] - b1), p10 = ex2_approx(v[2] - b0),
+                    p11 = ex2_approx(v[3] - b1);
+        l[nb][0] += p00 + p10;
+        l[nb][1] += p01 + p11;
+        pb[nb][0] = transpose_8x8(pack_h2(p00, p01));  // tokens 0..7: [token][head] -> [head][token], the B operand
+        pb[nb][1] = transpose_8x8(pack_h2(p10, p11));
       }
+#pragma unroll
+      for (int d = 0; d < kSteps; ++d) {
+        uint32_t a[4];
+        ldsm_x4_t(vbase + tile_off<HD>((mm >> 1) * 8 + rr, d * 2 + (mm & 1)), a[0], a[1], a[2], a[3]);
+#pragma unroll
+        for (int nb = 0; nb < NB; ++nb) mma16816(o[nb][d], a, pb[nb][0], pb[nb][1]);
+      }
+    }
+    // ---- merge the four warps: 2 and 3 into 0 and 1, 1 into 0.  (Three buffers: nobody writes one that may still be read.)
+#pragma unroll
+    for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int sh = 4; sh < 32; sh <<= 1) l[nb][e] += __shfl_xor_sync(0xffffffffu, l[nb][e], sh);
+    auto give = [&](float* buf) {
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int h = nb * 8 + t2 + e;
+#pragma unroll
+          for (int d = 0; d < kSteps; ++d) {
+            buf[h * kPitch + d * 16 + g] = o[nb][d][e];
+            buf[h * kPitch + d * 16 + g + 8] = o[nb][d][2 + e];
+          }
+          if (g == 0) {
+            buf[kHeads * kPitch + h] = m[nb][e];
+            buf[kHeads * kPitch + kHeads + h] = l[nb][e];
+          }
+        }
+    };
+    auto take = [&](const float* buf) {
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int h = nb * 8 + t2 + e;
+          const float om = buf[kHeads * kPitch + h], n = fmaxf(m[nb][e], om);
+          const float fa = m[nb][e] == -INFINITY ? 0.f : ex2_approx(m[nb][e] - n);
+          const float fb = om == -INFINITY ? 0.f : ex2_approx(om - n);
+          m[nb][e] = n;
+          l[nb][e] = l[nb][e] * fa + buf[kHeads * kPitch + kHeads + h] * fb;
+#pragma unroll
+          for (int d = 0; d < kSteps; ++d) {
+            o[nb][d][e] = o[nb][d][e] * fa + buf[h * kPitch + d * 16 + g] * fb;
+            o[nb][d][2 + e] = o[nb][d][2 + e] * fa + buf[h * kPitch + d * 16 + g + 8] * fb;
+          }
+        }
+    };
+    if (warp >= 2) give(merge + (warp - 2) * kBuf);
+    __syncthreads();
+    if (warp < 2) take(merge + warp * kBuf);
+    if (warp == 1) give(merge + 2 * kBuf);
+    __syncthreads();
+    if (warp == 0) {
+      take(merge + 2 * kBuf);
+      const int start = whole ? 0 : here - sg.first;             // position of the item's first tile
+      const int pieces = whole ? 1 : (start + sg.tiles - 1) / per - start / per + 1;
+      const bool alone = pieces == 1;
+      const int piece = alone ? 0 : int(blockIdx.x) - start / per;
+      if (!whole && sg.first == 0 && lane < G) *piece_count(scratch, sg.seq * nh + sg.kvh * G + lane, num_splits, HD) = pieces;
+#pragma unroll
+      for (int nb = 0; nb < NB; ++nb)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int h = nb * 8 + t2 + e;
+          if (h < G) {
+            const int head = sg.kvh * G + h;
+            if (alone) {
+              __half* dst = out + size_t(sg.seq) * ldo + size_t(head) * HD + g;
+              const float inv = l[nb][e] > 0.f ? 1.f / l[nb][e] : 0.f;
+#pragma unroll
+              for (int d = 0; d < kSteps; ++d) {
+                dst[d * 16] = __float2half_rn(o[nb][d][e] * inv);
+                dst[d * 16 + 8] = __float2half_rn(o[nb][d][2 + e] * inv);
+              }
+            } else {
+              float* dst = scratch + (size_t(sg.seq * nh + head) * num_splits + piece) * (HD + 2);
+#pragma unroll
+              for (int d = 0; d < kSteps; ++d) {
+                dst[d * 16 + g] = o[nb][d][e];
+                dst[d * 16 + g + 8] = o[nb][d][2 + e];
+              }
+              if (g == 0) {
+                dst[HD] = m[nb][e];
+                dst[HD + 1] = l[nb][e];
+              }
+            }
+          }
+        }
     }
   }
   cp_async_wait<0>();
-  l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-  l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-  l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-  l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
-  __syncthreads();                                       // every warp is done with its ring
-
-  // merge the four warps: smem as [warp][16 rows][HD] fp32 + [warp][16]{m, l}
-  float* mo = reinterpret_cast<float*>(smem);
-  float* mm = mo + kDecWarps * 16 * HD;
-  float* ml = mm + kDecWarps * 16;
-  {
-    const int r0 = lane >> 2, c = (lane & 3) * 2;
-    float* dst = mo + warp * 16 * HD;
-#pragma unroll
-    for (int n = 0; n < kNTilesO; ++n) {
-      dst[r0 * HD + n * 8 + c] = o[n][0];
-      dst[r0 * HD + n * 8 + c + 1] = o[n][1];
-      dst[(r0 + 8) * HD + n * 8 + c] = o[n][2];
-      dst[(r0 + 8) * HD + n * 8 + c + 1] = o[n][3];
-    }
-    if ((lane & 3) == 0) {
-      mm[warp * 16 + r0] = m0;
-      mm[warp * 16 + r0 + 8] = m1;
-      ml[warp * 16 + r0] = l0;
-      ml[warp * 16 + r0 + 8] = l1;
-    }
-  }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < G * HD; idx += blockDim.x) {
-    const int g = idx / HD, d = idx % HD;
-    float M = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kDecWarps; ++w) M = fmaxf(M, mm[w * 16 + g]);
-    float L = 0.f, acc = 0.f;
-#pragma unroll
-    for (int w = 0; w < kDecWarps; ++w) {
-      const float mw = mm[w * 16 + g];
-      const float f = mw == -INFINITY ? 0.f : exp2f(mw - M);
-      L += ml[w * 16 + g] * f;
-      acc += mo[(w * 16 + g) * HD + d] * f;
-    }
-    const int head = kvh * G + g;
-    if (num_splits == 1) {
-      out[size_t(seq) * ldo + size_t(head) * HD + d] = __float2half_rn(L > 0.f ? acc / L : 0.f);
-    } else {
-      float* dst = scratch + (size_t(seq * nh + head) * num_splits + split) * (HD + 2);
-      dst[d] = acc;
-      if (d == 0) {
-        dst[HD] = M;
-        dst[HD + 1] = L;
-      }
-    }
-  }
 }
 
+// Items that attn_decode_kernel cut in pieces.  grid (nh, sequences), HD threads.
 template <int HD>
-__global__ void attn_combine_kernel(const float* __restrict__ scratch, __half* __restrict__ out, int ldo, int nh,
-                                    int num_splits) {
+__global__ void attn_combine_kernel(float* __restrict__ scratch, __half* __restrict__ out, int ldo, int nh, int num_splits) {
   pdl_launch_dependents();
   pdl_wait();
   const int head = blockIdx.x, seq = blockIdx.y, d = threadIdx.x;
   const float* src = scratch + size_t(seq * nh + head) * num_splits * (HD + 2);
-  float M = -INFINITY;
-  for (int s = 0; s < num_splits; ++s) M = fmaxf(M, src[s * (HD + 2) + HD]);
-  float L = 0.f, acc = 0.f;
-  for (int s = 0; s < num_splits; ++s) {
+  // the records are read beside the count (num_splits >= 3: two are there, whatever they hold), not behind it
+  const int pieces = *piece_count(scratch, seq * nh + head, num_splits, HD);
+  const float m0 = src[HD], l0 = src[HD + 1], o0 = src[d], m1 = src[2 * HD + 2], l1 = src[2 * HD + 3], o1 = src[HD + 2 + d];
+  if (pieces == 1) return;                             // its CTA stored it
+  float M = fmaxf(m0, m1);
+  for (int s = 2; s < pieces; ++s) M = fmaxf(M, src[s * (HD + 2) + HD]);
+  const float f0 = m0 == -INFINITY ? 0.f : ex2_approx(m0 - M), f1 = m1 == -INFINITY ? 0.f : ex2_approx(m1 - M);
+  float L = l0 * f0 + l1 * f1, acc = o0 * f0 + o1 * f1;
+#pragma unroll 4
+  for (int s = 2; s < pieces; ++s) {
     const float ms = src[s * (HD + 2) + HD];
-    const float f = ms == -INFINITY ? 0.f : exp2f(ms - M);
+    const float f = ms == -INFINITY ? 0.f : ex2_approx(ms - M);
     L += src[s * (HD + 2) + HD + 1] * f;
     acc += src[s * (HD + 2) + d] * f;
   }
@@ -480,44 +647,66 @@ extern "C" int64_t zse_attn_decode_scratch_floats(int num_seqs, int nh, int hd, 
   return int64_t(num_seqs) * nh * max_splits * (hd + 2);
 }
 
-// Shared memory the decode kernel asks for, raised once per device (host work: not a stream operation).
-template <int HD, bool EXT>
+// Shared memory of the decode kernel: rings, three merge buffers, prefix sums of the lengths.
+template <int HD, int NB>
+constexpr int decode_smem(int num_seqs) {
+  return kDecWarps * kDecodeStages<HD, NB> * 2 * 16 * HD * 2 + 3 * (8 * NB * (HD + 4) + 2 * 8 * NB) * 4 + (num_seqs + 1) * 4;
+}
+constexpr int kDecMaxSeqs = 2048;                        // sequences of one call, bounded by the prefix sums' place
+
+// The attribute is raised once per device (host work: not a stream operation).
+template <int HD, bool EXT, int NB>
 static int prepare_decode() {
-  constexpr int ring = kDecWarps * kDecStages * 2 * 16 * HD * 2;
-  constexpr int merge = kDecWarps * 16 * HD * 4 + kDecWarps * 16 * 2 * 4;
-  constexpr int smem = ring > merge ? ring : merge;
   static bool attr[kMaxDevices] = {};
   const int dev_slot = current_device_slot();
   if (!attr[dev_slot]) {
-    if (cudaFuncSetAttribute(attn_decode_kernel<HD, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute(attn_decode_kernel<HD, EXT, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             decode_smem<HD, NB>(kDecMaxSeqs)) != cudaSuccess)
       return ZSE_ERR_LAUNCH;
     attr[dev_slot] = true;
   }
   return 0;
 }
 
-template <int HD, bool EXT>
+static int decode_sms() {
+  static int sms[kMaxDevices] = {};
+  const int d = current_device_slot();
+  if (sms[d] == 0) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, d) != cudaSuccess || n <= 0) n = 148;
+    sms[d] = n;
+  }
+  return sms[d];
+}
+
+template <int HD, bool EXT, int NB>
 static int launch_decode(const void* q, int ldq, const void* kv, const void* bt, int max_blocks, const void* lens,
                          void* out, int ldo, void* scratch, int num_seqs, int nh, int nkv, int block_size, int splits,
                          float scale, long long blk_stride, long long half_stride, float softcap, int window,
                          cudaStream_t st) {
-  constexpr int ring = kDecWarps * kDecStages * 2 * 16 * HD * 2;
-  constexpr int merge = kDecWarps * 16 * HD * 4 + kDecWarps * 16 * 2 * 4;
-  constexpr int smem = ring > merge ? ring : merge;
-  if (int rc = prepare_decode<HD, EXT>()) return rc;
-  dim3 grid(nkv, num_seqs, splits);
-  if (launch_pdl(attn_decode_kernel<HD, EXT>, grid, dim3(kDecWarps * 32), smem, st,
-                 reinterpret_cast<const __half*>(q), ldq, reinterpret_cast<const __half*>(kv),
-                 reinterpret_cast<const int*>(bt), max_blocks, reinterpret_cast<const int*>(lens),
-                 reinterpret_cast<__half*>(out), ldo, reinterpret_cast<float*>(scratch), nh, nkv, block_size, splits,
-                 scale * kLog2e, blk_stride, half_stride, softcap, window) != cudaSuccess)
-    return ZSE_ERR_LAUNCH;
-  if (splits > 1) {
-    if (launch_pdl(attn_combine_kernel<HD>, dim3(nh, num_seqs), dim3(HD), 0, st,
-                   reinterpret_cast<const float*>(scratch), reinterpret_cast<__half*>(out), ldo, nh,
-                   splits) != cudaSuccess)
+  if (int rc = prepare_decode<HD, EXT, NB>()) return rc;
+  const int tpb = block_size / 16;
+  int shift = 0;
+  while ((1 << shift) < tpb) ++shift;
+  if ((1 << shift) != tpb) shift = -1;
+  // cut: as many CTAs as the chip holds at once (rings of 48, 96 and 192 KB), each with the same share of the tiles
+  for (int s0 = 0; s0 < num_seqs; s0 += kDecMaxSeqs) {   // (one round in practice)
+    const int n = min(kDecMaxSeqs, num_seqs - s0);
+    const int fit = decode_sms() * (HD == 256 ? 1 : HD == 128 ? 2 : 4);
+    const int ctas = splits >= 3 ? min(fit, n * nkv * (splits - 1)) : n * nkv;         // (with few sequences most of the chip is left to the next kernel)
+    const __half* q0 = reinterpret_cast<const __half*>(q) + size_t(s0) * ldq;
+    __half* o0 = reinterpret_cast<__half*>(out) + size_t(s0) * ldo;
+    const int *bt0 = reinterpret_cast<const int*>(bt) + size_t(s0) * max_blocks, *l0 = reinterpret_cast<const int*>(lens) + s0;
+    if (launch_pdl(attn_decode_kernel<HD, EXT, NB>, dim3(ctas), dim3(kDecWarps * 32), size_t(decode_smem<HD, NB>(n)), st, q0,
+                   ldq, reinterpret_cast<const __half*>(kv), bt0, max_blocks, l0, o0, ldo, reinterpret_cast<float*>(scratch), n,
+                   nh, nkv, block_size, shift, splits, scale * kLog2e, blk_stride, half_stride, softcap,
+                   window) != cudaSuccess)
       return ZSE_ERR_LAUNCH;
+    if (splits >= 3) {
+      if (launch_pdl(attn_combine_kernel<HD>, dim3(nh, n), dim3(HD), 0, st, reinterpret_cast<float*>(scratch), o0, ldo, nh,
+                     splits) != cudaSuccess)
+        return ZSE_ERR_LAUNCH;
+    }
   }
   return 0;
 }
@@ -534,13 +723,19 @@ extern "C" int zse_attn_decode_ext(const void* q, int ldq, const void* kv_layer,
   if ((reinterpret_cast<uintptr_t>(kv_layer) & 15) || (blk_stride & 7) || (half_stride & 7)) return ZSE_ERR_ALIGN;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const bool ext = softcap > 0.f || window > 0;
-#define ZSE_DEC(HD_, EXT_)                                                                                           \
-  return launch_decode<HD_, EXT_>(q, ldq, kv_layer, block_tables, max_blocks, seq_lens, out, ldo, scratch, num_seqs, \
-                                  nh, nkv, block_size, num_splits, scale, blk_stride, half_stride, softcap, window, st)
-  if (hd == 128) { if (ext) ZSE_DEC(128, true); ZSE_DEC(128, false); }
-  if (hd == 64) { if (ext) ZSE_DEC(64, true); ZSE_DEC(64, false); }
-  if (hd == 256) ZSE_DEC(256, true);
+#define ZSE_DEC_NB(HD_, EXT_, NB_)                                                                                       \
+  return launch_decode<HD_, EXT_, NB_>(q, ldq, kv_layer, block_tables, max_blocks, seq_lens, out, ldo, scratch, num_seqs, \
+                                       nh, nkv, block_size, num_splits, scale, blk_stride, half_stride, softcap, window, st)
+#define ZSE_DEC(HD_, EXT_)                          \
+  {                                                 \
+    if (nh / nkv <= 8) ZSE_DEC_NB(HD_, EXT_, 1);    \
+    ZSE_DEC_NB(HD_, EXT_, 2);                       \
+  }
+  if (hd == 128) { if (ext) ZSE_DEC(128, true) ZSE_DEC(128, false) }
+  if (hd == 64) { if (ext) ZSE_DEC(64, true) ZSE_DEC(64, false) }
+  if (hd == 256) ZSE_DEC(256, true)
 #undef ZSE_DEC
+#undef ZSE_DEC_NB
   return ZSE_ERR_SHAPE;
 }
 
@@ -641,9 +836,12 @@ extern "C" int zse_attn_decode_static_setup(void) {
   int err = 0;
   static_scratch(&err);
   if (err) return err;
-  if (int rc = prepare_decode<128, false>()) return rc;
-  if (int rc = prepare_decode<64, false>()) return rc;
-  return prepare_decode<256, true>();
+  if (int rc = prepare_decode<128, false, 1>()) return rc;
+  if (int rc = prepare_decode<128, false, 2>()) return rc;
+  if (int rc = prepare_decode<64, false, 1>()) return rc;
+  if (int rc = prepare_decode<64, false, 2>()) return rc;
+  if (int rc = prepare_decode<256, true, 1>()) return rc;
+  return prepare_decode<256, true, 2>();
 }
 
 extern "C" int zse_attn_decode_static(const void* q, int ldq, const void* kv_layer, const void* block_tables,
