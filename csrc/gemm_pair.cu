@@ -511,8 +511,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const PairArgs a) {
 }
 
 // ---- plan ------------------------------------------------------------------------------------------------------------------
-// Tokens per unit and K splits.  A unit costs spp chunks of 8 MMAs (nt / 2 cycles each on a pair, but not less than a chunk
-// takes to arrive and be dequantised) and a fixed part for the hand-over of the accumulator; all pairs work in rounds.
+// Tokens per unit and K splits.  A unit costs spp chunks (8 MMAs of nt / 2 cycles on a pair and what surrounds them, but not
+// less than a chunk takes to arrive and be dequantised) and a fixed part for the hand-over of the accumulator; all pairs work in
+// rounds.
 // More token tiles than necessary can be right when they fill the last round better; K splits (planes, where the consumer
 // adds them) fill the machine when there are fewer units than pairs, at the price of writing and reading a plane each.
 struct PairPlan {
@@ -533,8 +534,8 @@ static PairPlan plan_pair(int M, int N, int K, bool planes_ok, int n_tiles, int 
       const int spp = (k_stages + ks - 1) / ks;
       const long units = long(n_pairs) * m_tiles * ks;
       const long rounds = (units + workers - 1) / workers;
-      const double chunk = max(4.0 * nt + 60.0, 330.0);
-      double cost = double(rounds) * (spp * chunk + 1500.0);
+      const double chunk = max(6.6 * nt, 950.0);               // cycles, from timed layers of 72 to 512 tokens
+      double cost = double(rounds) * (spp * chunk + 3000.0);
       cost += double(ks - 1) * double(M) * N * 8.0 / 4000.0;
       if (best_cost < 0 || cost < best_cost) {
         best_cost = cost;

@@ -93,6 +93,7 @@ struct W4Args {
   long long* timing;       // debug builds (ZSE_W4_TIMING): per-role cycle counters, else unused
   PushTable push;          // kEpiPushF16: where the partial tiles go (every rank's inbox over NVLink)
   SpTable sp;              // kEpiScatterF16: where the partial tiles go (the owner of each 64-row block)
+  GatherWait gather;       // the activations are a gathered buffer: wait for the row blocks of this CTA's token tile
 };
 
 __device__ __forceinline__ void multimem_st_v4(void* mc_ptr, const uint4& v) {
@@ -110,6 +111,35 @@ __device__ __forceinline__ void red_add_relaxed_sys(uint32_t* p, uint32_t v) {
 __device__ __forceinline__ void red_add_release_sys(uint32_t* p, uint32_t v) {
   asm volatile("red.release.sys.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+__device__ __forceinline__ uint32_t w4_ld_acquire_sys(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// All-gather in the prologue: the rows of token tile [t0, t0 + nt) were written into this GPU's memory by their
+// owners (other GPUs, plain or multicast stores); a row block is complete when its flag holds the pass epoch.  One
+// thread waits (bounded), then orders those writes before the TMA loads it is about to issue (async proxy).
+__device__ __forceinline__ bool gather_wait_tile(const GatherWait& g, int t0, int nt, int M, volatile int* abort_flag,
+                                                 Status* st) {
+  const uint32_t want = *reinterpret_cast<const volatile uint32_t*>(g.epoch);
+  bool ok = true;
+  for (int t = t0; t < t0 + nt && t < M && ok; t += kSpRowBlock) {
+    const uint32_t* f = g.flags + t / kSpRowBlock;
+    if (w4_ld_acquire_sys(f) == want) continue;
+    SpinClock clk;
+    while (w4_ld_acquire_sys(f) != want) {
+      if (clk.expired(0x3F) || ((clk.spins & 0x3F) == 0 && *abort_flag)) {
+        report(st, kPeerTimeout, 36, unsigned(t / kSpRowBlock));
+        *abort_flag = 1;
+        ok = false;
+        break;
+      }
+    }
+  }
+  asm volatile("fence.proxy.async;" ::: "memory");
+  return ok;
+}
+
 // Nibble order inside every 32-bit word of a chunk (fixed by repack_w4): positions 0..7 hold the K elements
 // e0,e2,e4,e6,e1,e3,e5,e7 so that masking with 0x000f000f yields the adjacent pair (e0,e1) as a half2.
 __device__ __forceinline__ void dequant_word(uint32_t w, __half2 s2, __half2 z2, uint32_t* out4) {
@@ -417,7 +447,10 @@ gemm_w4_kernel(const __grid_constant__ CUtensorMap tmap_x, const W4Args a) {
       int issued = 0, s = 0;
       uint32_t ph = 1;
       pdl_wait();                                        // the activations come from the previous kernel
-      for (int kk = 0; kk < n_k; ++kk) {
+      bool gathered = true;
+      if (a.gather.flags != nullptr)
+        gathered = gather_wait_tile(a.gather, blockIdx.y * NT, NT, a.M, abort_flag, a.status);
+      for (int kk = 0; kk < n_k && gathered; ++kk) {
         if (kk >= SX) {
           // tied: the commit that ends the pair holding this stage's last chunk frees the stage as well
           uint64_t* freed = kTied ? &bars->pair_done[s / (CPS / R)] : &bars->x_empty[s];
@@ -797,11 +830,11 @@ static int launch_w4(const CUtensorMap& tx, const W4Args& a, dim3 grid, cudaStre
 template <int NT, int R, bool DUAL = false>
 static int launch_w4_epi(int epilogue, const CUtensorMap& tx, const W4Args& a, dim3 grid, cudaStream_t st) {
   if (epilogue == kEpiPushF16) return launch_w4<NT, R, kEpiPushF16, DUAL>(tx, a, grid, st);
-  if constexpr (NT >= 128) {         // more than 64 rows: only the exchanges with other ranks come here (gemm_pair.cu)
+  if (epilogue == kEpiF16) return launch_w4<NT, R, kEpiF16, DUAL>(tx, a, grid, st);
+  if (epilogue == kEpiSwiGLU) return launch_w4<NT, R, kEpiSwiGLU, DUAL>(tx, a, grid, st);
+  if constexpr (NT >= 128) {         // the row-block exchange is for passes of many rows; their planes come from gemm_pair.cu
     if (epilogue == kEpiScatterF16) return launch_w4<NT, R, kEpiScatterF16, DUAL>(tx, a, grid, st);
   } else {
-    if (epilogue == kEpiF16) return launch_w4<NT, R, kEpiF16, DUAL>(tx, a, grid, st);
-    if (epilogue == kEpiSwiGLU) return launch_w4<NT, R, kEpiSwiGLU, DUAL>(tx, a, grid, st);
     if (epilogue == kEpiPartialF32) return launch_w4<NT, R, kEpiPartialF32, DUAL>(tx, a, grid, st);
   }
   return ZSE_ERR_SHAPE;
@@ -896,6 +929,16 @@ static bool takes_small(int M, int K, int epilogue, int k_split) {
   return g_w4_mode == 0 && gemm_w4_small_takes(M, K) && (epilogue == kEpiPartialF32 || k_split <= 0);
 }
 
+// More than 64 tokens: gemm_pair.cu, except for narrow layers whose epilogue needs the whole sum.  They leave most pairs without
+// work, and a cluster along K of this file's wide CTA adds the parts on chip.  The line lies between 14 pairs of tiles (Gemma-2 9B
+// o_proj, 128 tokens: 17.4 us here, 23.4 there; down_proj 35.7, 53.2) and 18 (7B QKV, 128 tokens: 27.6 us here, 22.5 there), and at
+// 256 tokens (o_proj, 320 tokens: 27.6, 24.6).
+static bool takes_pair(int M, int N, int epilogue, int sm_count) {
+  if (M <= 64) return false;
+  const int pairs = ((epilogue == kEpiSwiGLU ? (N / 2 + 63) / 64 : (N + kTileN - 1) / kTileN) + 1) / 2;
+  return epilogue == kEpiPartialF32 || M > 256 || 5 * pairs > sm_count / 2;
+}
+
 static int run_gemm_w4(const void* w_tiled, const void* x, int x_rows_cap, const void* bias, void* out, int M, int N,
                        int K, int ldo, int epilogue, int k_split, void* status, void* stream, const PushTable* push,
                        int* ctas_out, const SpTable* sp = nullptr, const GatherWait* gather = nullptr) {
@@ -912,7 +955,7 @@ static int run_gemm_w4(const void* w_tiled, const void* x, int x_rows_cap, const
   if (push == nullptr && takes_small(M, K, epilogue, k_split))
     return gemm_w4_small_run(w_tiled, x, bias, out, M, N, K, ldo, epilogue, k_split, nullptr,
                              reinterpret_cast<cudaStream_t>(stream));
-  if (push == nullptr && sp == nullptr && M > 64)       // (a K split of a fused epilogue is a plan of the kernels below)
+  if (push == nullptr && sp == nullptr && takes_pair(M, N, epilogue, sm_count))
     return gemm_pair_run(false, w_tiled, x, x_rows_cap, bias, out, M, N, K, ldo, epilogue, k_split, gather,
                          reinterpret_cast<Status*>(status), reinterpret_cast<cudaStream_t>(stream));
   const int k_stages = K / kW4StageK;
@@ -926,7 +969,8 @@ static int run_gemm_w4(const void* w_tiled, const void* x, int x_rows_cap, const
   CUtensorMap tx;
   if (int rc = get_tmap(x, uint64_t(max(x_rows_cap, M)), uint64_t(K), uint32_t(nt), &tx)) return rc;
   W4Args a{reinterpret_cast<const uint8_t*>(w_tiled), reinterpret_cast<const __half*>(bias), out, M, N, K, ldo,
-           k_stages, spp, cluster, reinterpret_cast<Status*>(status), g_w4_timing, PushTable{}, SpTable{}};
+           k_stages, spp, cluster, reinterpret_cast<Status*>(status), g_w4_timing, PushTable{}, SpTable{},
+           gather != nullptr ? *gather : GatherWait{nullptr, nullptr}};
   if (push != nullptr) a.push = *push;
   if (sp != nullptr) a.sp = *sp;
   dim3 grid(n_tiles / R, (M + nt - 1) / nt, ks);
