@@ -5,6 +5,9 @@
 // Computed transposed ("swap AB"): UMMA M (128) runs over weight rows, UMMA N (16..256) over tokens, so a decode step
 // with a few tokens fills the TMEM lanes and the weight stream is read exactly once.
 //
+// Which passes come here: 9 to 64 tokens (narrow CTA), narrow layers of up to 256 tokens and what exchanges rows with other ranks
+// (wide CTA).  Up to 8 tokens take gemm_w4_small.cu, all else above 64 gemm_pair.cu (takes_small, takes_pair).
+//
 // Data flow of one CTA (608 threads):
 //   warp 0      streams 8704-byte weight chunks (8192 B nibbles + 128 x {scale, zero}) with 1-D bulk TMA copies
 //               into a deep ring (up to 12 chunks in flight: this ring is what hides HBM latency);
