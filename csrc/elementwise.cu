@@ -304,7 +304,10 @@ __global__ void rope_kv_write_kernel(__half* __restrict__ qkv, __half* __restric
 // (i .. i+7 and their partners half a head away): the CTA computes the token's sines and cosines once, then its threads walk
 // the heads with two 16-byte loads and two 16-byte stores each.  The one-CTA-per-head form above spends 271 us on a prefill pass
 // of 8 k tokens of the 14B shape (229 k CTAs of 64 threads, 2-byte accesses, a sincosf per element and head).
-__global__ void __launch_bounds__(256)
+// blockDim.x is a multiple of hd / 16: threads left over would walk heads that others rotate in place.
+constexpr int kRopeThreads = 256;
+
+__global__ void __launch_bounds__(kRopeThreads)
 rope_kv_write_vec_kernel(__half* __restrict__ qkv, __half* __restrict__ kv_layer, const int* __restrict__ positions,
                          const long long* __restrict__ slots, const float* __restrict__ inv_freq, int nh, int nkv,
                          int hd, int block_size) {
@@ -482,8 +485,9 @@ extern "C" int zse_rope_kv_write(void* qkv, void* kv_layer, const void* position
   if (hd % 2 || hd > 2048 || rotary_dim % 2 || rotary_dim > hd || (hd - rotary_dim) % 2) return ZSE_ERR_SHAPE;
   if (planes == nullptr && rotary_dim == hd && hd % 16 == 0 && hd <= 512 &&
       (reinterpret_cast<uintptr_t>(qkv) & 15) == 0 && (reinterpret_cast<uintptr_t>(kv_layer) & 15) == 0)
-    return launch_pdl(rope_kv_write_vec_kernel, dim3(M), dim3(256), 0, ST(stream), reinterpret_cast<__half*>(qkv),
-                      reinterpret_cast<__half*>(kv_layer), reinterpret_cast<const int*>(positions),
+    return launch_pdl(rope_kv_write_vec_kernel, dim3(M), dim3(kRopeThreads / (hd / 16) * (hd / 16)), 0, ST(stream),
+                      reinterpret_cast<__half*>(qkv), reinterpret_cast<__half*>(kv_layer),
+                      reinterpret_cast<const int*>(positions),
                       reinterpret_cast<const long long*>(slots), reinterpret_cast<const float*>(inv_freq), nh, nkv, hd,
                       block_size) == cudaSuccess ? 0 : ZSE_ERR_LAUNCH;
   dim3 grid(M, nh + 2 * nkv);

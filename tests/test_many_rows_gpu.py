@@ -57,6 +57,32 @@ def test_post_norm(ops, H, scaled, out):
     assert (r1 - r2).abs().max() < 1e-5 and _close(o1, o2, 1e-5)      # the residual is fp32: sums of squares in another order
 
 
+@pytest.mark.parametrize("hd,nh,nkv", [(96, 32, 32), (160, 32, 8), (80, 32, 32), (48, 60, 15), (512, 5, 1), (16, 3, 1)])
+@pytest.mark.parametrize("M", [1, 33])
+def test_rotation_of_heads_that_leave_threads_over(ops, hd, nh, nkv, M):
+    """hd / 16 threads a head: where that does not divide the CTA, and there are more heads than fit it at once."""
+    bs, half = 16, hd // 2
+    g = torch.Generator(device="cuda").manual_seed(hd + M)
+    qkv = torch.randn(M, (nh + 2 * nkv) * hd, device="cuda", generator=g).half()
+    pos = torch.randint(0, 64, (M,), dtype=torch.int32, device="cuda", generator=g)
+    slots = torch.randperm(64, device="cuda", generator=g)[:M].to(torch.int64)
+    freqs = 1e4 ** (-torch.arange(half, device="cuda").float() / half)
+    kv = torch.full((4, 2, nkv, bs, hd), 7.0, dtype=torch.float16, device="cuda")
+    x = qkv.double().view(M, nh + 2 * nkv, hd)
+    ops.rope_kv_write(qkv, kv, pos, slots, freqs, M, nh, nkv, hd, bs)
+    torch.cuda.synchronize()
+    ang = pos.double()[:, None] * freqs.double()
+    c, s = ang.cos()[:, None], ang.sin()[:, None]
+    a, b = x[:, : nh + nkv, :half], x[:, : nh + nkv, half:]
+    turned = torch.cat([a * c - b * s, b * c + a * s], -1)
+    # one rounding to fp16, and angles of up to 64 in fp32 (64 * 2^-24) times what is rotated
+    close = lambda got, want: bool(((got.double() - want).abs() <= UNIT / 2 * want.abs() + 1e-4).all())
+    assert close(qkv.view(M, -1, hd)[:, : nh + nkv], turned)
+    blk, off = slots // bs, slots % bs
+    assert close(kv[blk, 0, :, off], turned[:, nh:]) and close(kv[blk, 1, :, off], x[:, nh + nkv:])
+    assert int((kv != 7).any(-1).any(2).any(1).sum()) == M
+
+
 @pytest.mark.parametrize("hd,nh,nkv,k_is_v,norm_v", [(256, 16, 8, False, False), (8, 3, 1, False, False), (64, 4, 2, True, True),
                                                      (512, 8, 1, False, True), (200, 2, 2, False, False)])
 def test_head_norms(ops, hd, nh, nkv, k_is_v, norm_v):
