@@ -66,12 +66,85 @@ __device__ __forceinline__ void small_mma(float (&d)[4], uint32_t a0, uint32_t a
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// A sum that came out infinite or NaN, again with weights as the other kernels have them (fp16 of scale * q + minimum): scale *
+// sum(q x) + minimum * sum(x) is inf - inf, or 0 * inf, where an infinite activation times the weight is infinite.  Sums of finite
+// activations are finite (products of fp16 numbers, fp32), so nobody else comes here.  One row of a tile, K groups from `chunk` on.
+__device__ __forceinline__ float small_not_finite(const uint8_t* chunk, int row, int groups, const __half* x) {
+  float y = 0.f;
+#pragma unroll 1
+  for (int k = 0; k < groups; ++k, chunk += kW4ChunkBytes) {
+    const __half2 sz = *reinterpret_cast<const __half2*>(chunk + 8192 + row * 4);
+#pragma unroll 1
+    for (int i = 0; i < 16; ++i, x += 8) {                     // eight columns a word
+      const uint32_t u = *reinterpret_cast<const uint32_t*>(chunk + (i >> 2) * 2048 + row * 16 + (i & 3) * 4);
+      for (int c = 0; c < 8; ++c) {
+        const int q = (u >> ((c >> 1) * 4 + (c & 1) * 16)) & 15;
+        y = fmaf(__half2float(__hfma(__int2half_rn(q), __low2half(sz), __high2half(sz))), __half2float(x[c]), y);
+      }
+    }
+  }
+  return y;
+}
+
 template <int EPI>
 __global__ void __launch_bounds__(kSmallThreads, 1) gemm_w4_small_kernel(const SmallArgs a) {
   extern __shared__ float red[];                               // [warps][8 columns][kSmallPitch]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   pdl_launch_dependents();
+  constexpr bool kPairs = EPI == kEpiSwiGLU || EPI == kEpiQkvRope;
+  constexpr float kMaxFloat = 3.402823466e38f;
+  __shared__ uint32_t odd_tokens;                              // tokens with a sum that is not finite
+  if (threadIdx.x == 0) odd_tokens = 0;
+  // rows j and 32 + j of a half tile, the two of a gate/up or rotation pair
+  auto store2 = [&](int item, int tok, int j, float va, float vb) {
+    const int tile = item >> 1, h32 = (item & 1) * 32;         // (these epilogues have no K splits: an item is a half tile)
+    if (EPI == kEpiSwiGLU) {
+      const int n = tile * 64 + h32 + j;
+      if (n < a.N / 2)
+        reinterpret_cast<__half*>(a.out)[size_t(tok) * a.ldo + n] = __float2half_rn(clamp_f16(silu_f(va) * vb));
+      return;
+    }
+    // a tile is a head of 128: q heads, k heads, v heads; dims d and d + 64 rotate together
+    const SmallRope& rp = a.rope;
+    const int d = h32 + j;
+    if (a.bias != nullptr) {
+      va += __half2float(a.bias[tile * 128 + d]);
+      vb += __half2float(a.bias[tile * 128 + 64 + d]);
+    }
+    if (tile < rp.nh + rp.nkv) {
+      const int pos = min(max(rp.positions[tok], 0), rp.max_position - 1);
+      const float2 cs = rp.cos_sin[size_t(pos) * 64 + d];
+      const float ra = va * cs.x - vb * cs.y, rb = vb * cs.x + va * cs.y;
+      va = ra, vb = rb;
+    }
+    __half* dst = nullptr;
+    if (tile < rp.nh) {
+      dst = reinterpret_cast<__half*>(a.out) + size_t(tok) * a.ldo + tile * 128;
+    } else {
+      const long long slot = rp.slots[tok];
+      if (slot >= 0) {
+        const bool is_v = tile >= rp.nh + rp.nkv;
+        const int kvh = tile - rp.nh - (is_v ? rp.nkv : 0);
+        const long long blk = slot / rp.block_size, off = slot % rp.block_size;
+        dst = rp.kv_layer + (((blk * 2 + (is_v ? 1 : 0)) * rp.nkv + kvh) * rp.block_size + off) * 128;
+      }
+    }
+    if (dst != nullptr) {
+      dst[d] = __float2half_rn(clamp_f16(va));
+      dst[64 + d] = __float2half_rn(clamp_f16(vb));
+    }
+  };
+  auto store1 = [&](int item, int tok, int row, float s) {
+    const int z = item / a.n_half, half = item - z * a.n_half;
+    const int n = (half >> 1) * 128 + (half & 1) * 32 + (row < 32 ? row : row + 32);
+    if (n >= a.N) return;
+    if (EPI == kEpiF16)
+      reinterpret_cast<__half*>(a.out)[size_t(tok) * a.ldo + n] =
+          __float2half_rn(clamp_f16(s + (a.bias != nullptr ? __half2float(a.bias[n]) : 0.f)));
+    else
+      reinterpret_cast<float*>(a.out)[(size_t(z) * a.M + tok) * a.ldo + n] = s;
+  };
 
   uint4 w[8];                                                  // [16-row block][row g, row g + 8] of the group in flight
   uint32_t sz[8];
@@ -120,7 +193,6 @@ __global__ void __launch_bounds__(kSmallThreads, 1) gemm_w4_small_kernel(const S
   };
   if (f_item < a.items) fetch_x();
   for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
-    const int z = item / a.n_half, half = item - z * a.n_half;
     float y[4][4];
 #pragma unroll
     for (int st = 0; st < 4; ++st)
@@ -186,67 +258,50 @@ __global__ void __launch_bounds__(kSmallThreads, 1) gemm_w4_small_kernel(const S
 #pragma unroll
       for (int i = 0; i < 4; ++i) mine[(2 * t + (i & 1)) * kSmallPitch + st * 16 + g + (i >> 1) * 8] = y[st][i];
     __syncthreads();
-    const int tile = half >> 1, h32 = (half & 1) * 32;
     auto total = [&](int col, int row) {
       float s = 0.f;
       for (int i = 0; i < warps; ++i) s += red[(i * 8 + col) * kSmallPitch + row];
       return s;
     };
-    if (EPI == kEpiSwiGLU || EPI == kEpiQkvRope) {
+    // sums of a thread's outputs (rows j and 32 + j together where the epilogue needs both) that are not finite are noted
+    // for the end, so that the loop carries no registers for them
+    if (kPairs) {
       for (int e = threadIdx.x; e < a.M * 32; e += blockDim.x) {
         const int tok = e >> 5, j = e & 31;
-        float va = total(tok, j), vb = total(tok, 32 + j);
-        if (EPI == kEpiSwiGLU) {
-          const int n = tile * 64 + h32 + j;
-          if (n < a.N / 2)
-            reinterpret_cast<__half*>(a.out)[size_t(tok) * a.ldo + n] = __float2half_rn(clamp_f16(silu_f(va) * vb));
-        } else {
-          // a tile is a head of 128: q heads, k heads, v heads; dims d and d + 64 rotate together
-          const SmallRope& rp = a.rope;
-          const int d = h32 + j;
-          if (a.bias != nullptr) {
-            va += __half2float(a.bias[tile * 128 + d]);
-            vb += __half2float(a.bias[tile * 128 + 64 + d]);
-          }
-          if (tile < rp.nh + rp.nkv) {
-            const int pos = min(max(rp.positions[tok], 0), rp.max_position - 1);
-            const float2 cs = rp.cos_sin[size_t(pos) * 64 + d];
-            const float ra = va * cs.x - vb * cs.y, rb = vb * cs.x + va * cs.y;
-            va = ra, vb = rb;
-          }
-          __half* dst = nullptr;
-          if (tile < rp.nh) {
-            dst = reinterpret_cast<__half*>(a.out) + size_t(tok) * a.ldo + tile * 128;
-          } else {
-            const long long slot = rp.slots[tok];
-            if (slot >= 0) {
-              const bool is_v = tile >= rp.nh + rp.nkv;
-              const int kvh = tile - rp.nh - (is_v ? rp.nkv : 0);
-              const long long blk = slot / rp.block_size, off = slot % rp.block_size;
-              dst = rp.kv_layer + (((blk * 2 + (is_v ? 1 : 0)) * rp.nkv + kvh) * rp.block_size + off) * 128;
-            }
-          }
-          if (dst != nullptr) {
-            dst[d] = __float2half_rn(clamp_f16(va));
-            dst[64 + d] = __float2half_rn(clamp_f16(vb));
-          }
-        }
+        const float va = total(tok, j), vb = total(tok, 32 + j);
+        if (!(fabsf(va) + fabsf(vb) <= kMaxFloat)) atomicOr(&odd_tokens, 1u << tok);
+        store2(item, tok, j, va, vb);
       }
     } else {
       for (int e = threadIdx.x; e < a.M * 64; e += blockDim.x) {
         const int tok = e >> 6, row = e & 63;
-        const int n = tile * 128 + h32 + (row < 32 ? row : row + 32);
-        if (n < a.N) {
-          const float s = total(tok, row);
-          if (EPI == kEpiF16)
-            reinterpret_cast<__half*>(a.out)[size_t(tok) * a.ldo + n] =
-                __float2half_rn(clamp_f16(s + (a.bias != nullptr ? __half2float(a.bias[n]) : 0.f)));
-          else
-            reinterpret_cast<float*>(a.out)[(size_t(z) * a.M + tok) * a.ldo + n] = s;
-        }
+        const float s = total(tok, row);
+        if (!(fabsf(s) <= kMaxFloat)) atomicOr(&odd_tokens, 1u << tok);
+        store1(item, tok, row, s);
       }
     }
     __syncthreads();
+  }
+  if (odd_tokens == 0) return;
+#pragma unroll 1
+  for (int item = blockIdx.x; item < a.items; item += gridDim.x) {
+    const int z = item / a.n_half, half = item - z * a.n_half, k0 = z * a.spp, groups = min(a.k_stages, k0 + a.spp) - k0;
+    const uint8_t* chunk = a.w + (size_t(half >> 1) * a.k_stages + k0) * kW4ChunkBytes;
+    constexpr int rows = kPairs ? 32 : 64;
+#pragma unroll 1
+    for (int e = threadIdx.x; e < a.M * rows; e += blockDim.x) {
+      const int tok = e / rows, row = e % rows;
+      if (((odd_tokens >> tok) & 1) == 0) continue;
+      const __half* x = a.x + size_t(tok) * a.K + k0 * kW4StageK;
+      const int r = (half & 1) * 32 + (row < 32 ? row : row + 32);
+      const float va = small_not_finite(chunk, r, groups, x);
+      if (kPairs) {
+        const float vb = small_not_finite(chunk, r + 64, groups, x);
+        if (!(fabsf(va) + fabsf(vb) <= kMaxFloat)) store2(item, tok, row, va, vb);
+      } else if (!(fabsf(va) <= kMaxFloat)) {
+        store1(item, tok, row, va);
+      }
+    }
   }
 }
 

@@ -107,3 +107,31 @@ def test_small_qkv_rope(ops, M, nh, nkv, K):
         blk, off = divmod(int(slots[m]), bs)
         assert _rel(kv[blk, 0, :, off], turned[m, nh:]) < 6e-4 and _rel(kv[blk, 1, :, off], y[m, nh + nkv:]) < 6e-4
     assert int((kv != 7).any(-1).any(2).any(1).sum()) == M - 1      # nothing else was written
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 256, 640), (2, 4864, 256), (8, 200, 2176)])
+def test_small_infinite_activation(ops, M, N, K):
+    """An infinite activation times a weight that is not zero is infinite, of the product's sign: 65504 where outputs are fp16."""
+    p, _ = _part(N, K, K)
+    q = np.stack([p["data"] & 15, p["data"] >> 4], -1).reshape(N, -1, 128)
+    w = (q * p["scales"][..., None].astype(np.float32) + p["zeros"][..., None].astype(np.float32)).astype(np.float16).reshape(N, K)
+    x = (torch.randn(M, K, device="cuda") * 0.5).half()
+    at = [(37 * m + 5) % K for m in range(M)]
+    for m in range(0, M, 2):                                  # the other tokens are finite
+        x[m, at[m]] = float("inf") if m % 4 == 0 else float("-inf")
+    out = torch.zeros(M, N, dtype=torch.float16, device="cuda")
+    ops.linear(ops.make_linear([p], K, 128), x, M, out)
+    planes = torch.zeros(8, M, N, dtype=torch.float32, device="cuda")
+    n = ops.linear_partial(ops.make_linear([p], K, 128), x, M, planes)
+    torch.cuda.synchronize()
+    ops.check()
+    want = x.double() @ torch.from_numpy(w).cuda().double().T
+    for m in range(M):
+        if m % 2:
+            assert torch.isfinite(out[m]).all() and _rel(planes[:n, m].double().sum(0), want[m]) < 5e-4
+            continue
+        col = torch.from_numpy(w[:, at[m]]).cuda().float()
+        sign = torch.sign(col) * torch.sign(x[m, at[m]].float())
+        ok = col != 0
+        assert int(ok.sum()) > N // 2 and torch.equal(out[m][ok].float(), 65504 * sign[ok])
+        assert torch.equal(planes[:n, m].sum(0)[ok], float("inf") * sign[ok])
