@@ -111,7 +111,7 @@ headnorm_rope_rows_kernel(__half* __restrict__ qkv, int ld, __half* __restrict__
   const float pos = float(positions[t]);
   for (int i = threadIdx.x; i < half; i += blockDim.x) {
     const float f = freqs[i];
-    float s = 0.f, c = 1.f;                                    // frequency 0: the pair passes through
+    float s = 0.f, c = 2.f;                                    // frequency 0 (no cosine): the pair passes through as it is
     if (f != 0.f) sincosf(pos * f, &s, &c);
     sin_t[i] = s, cos_t[i] = c;
   }
@@ -168,7 +168,7 @@ headnorm_rope_rows_kernel(__half* __restrict__ qkv, int ld, __half* __restrict__
         if (!is_v) {
           const float s = sin_t[i + k], c = cos_t[i + k];
           const float rx = x[k] * c - y[k] * s, ry = y[k] * c + x[k] * s;
-          x[k] = rx, y[k] = ry;
+          if (c != 2.f) x[k] = rx, y[k] = ry;
         }
       }
       *reinterpret_cast<uint2*>(dst + i) = make_uint2(pack_half2(clamp_f16(x[0]), clamp_f16(x[1])),

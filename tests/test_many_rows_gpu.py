@@ -108,6 +108,32 @@ def test_head_norms(ops, hd, nh, nkv, k_is_v, norm_v):
     assert torch.equal(got[0][1] == 7, got[1][1] == 7)
 
 
+def test_pairs_that_do_not_rotate_pass_infinities_through(ops):
+    """Frequency 0: an infinite or NaN partner does not reach the other element of the pair."""
+    hd, nh, nkv, bs, M, step = 64, 2, 1, 16, 300, 150
+    qkv = torch.randn(M, (nh + 2 * nkv) * hd, device="cuda").half()
+    qkv[::3, 20], qkv[1::3, 20 + hd // 2], qkv[2::3, hd + 25] = float("inf"), float("nan"), float("-inf")
+    qkv[::2, 2 * hd + 30] = float("inf")
+    pos = torch.arange(M, dtype=torch.int32, device="cuda")
+    slots = torch.arange(M, device="cuda")
+    freqs = 1e4 ** (-torch.arange(hd // 2, device="cuda").float() / (hd // 2))
+    freqs[hd // 4:] = 0
+    got = []
+    for n in (M, step):
+        q, kv = qkv.clone(), torch.zeros(20, 2, nkv, bs, hd, dtype=torch.float16, device="cuda")
+        for i in range(0, M, n):
+            ops.headnorm_rope_kv_write(q[i:i + n], kv, pos[i:i + n], slots[i:i + n], freqs, None, None, False, False, 1e-6, n, nh,
+                                       nkv, hd, bs)
+        got.append((q, kv))
+    torch.cuda.synchronize()
+    still = torch.arange(hd, device="cuda") % (hd // 2) >= hd // 4
+    heads = qkv[:, : nh * hd].view(M, nh, hd)[:, :, still].float()
+    heads = torch.nan_to_num(heads, nan=-65504.0).clamp(-65504, 65504)        # (what the clamp before the store makes of them)
+    for q, kv in got:
+        assert torch.equal(q[:, : nh * hd].view(M, nh, hd)[:, :, still].float(), heads)
+    assert _close(got[0][1], got[1][1], 2e-3)
+
+
 @pytest.mark.parametrize("M,I", [(1, 8), (3, 14336), (70, 264), (5, 2056), (4, 20)])
 @pytest.mark.parametrize("gelu", [False, True])
 def test_glu(ops, M, I, gelu):
