@@ -8,7 +8,8 @@
 //                       reference reads them once per query head, kernels.py:524-671).  One grid of as many CTAs as fit; each
 //                       takes an equal run of 16-token tiles over all sequences and kv heads, its four warps
 //                       stream tiles through private 3-stage cp.async rings that run on from one item into the next (no CTA
-//                       barriers in the main loop), keep an online softmax in registers and merge at the end of an item.
+//                       barriers in the main loop), keep an online softmax in registers and give it to shared memory at the end
+//                       of an item, where all threads add it up.
 // attn_prefill_kernel - causal attention of a chunk of query tokens against everything already in the cache
 //                       (earlier chunks included), flash-attention style: 64 query rows per CTA, 64-token KV tiles,
 //                       online softmax.  Serves prefill, chunked prefill and speculative verification
@@ -91,6 +92,12 @@ __device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
 // Tokens are the 16 rows of the products and query heads their 8 columns (S^T = K Q^T, O^T = V^T P^T; the probabilities change
 // sides with movmatrix).  With heads as the rows, half of every product, every exponential and half of the accumulators were for
 // heads that do not exist (groups of 2 to 8): 385 instructions a tile and 164 registers.
+//
+// With few sequences a launch is all start and end, and in a layer the instructions come from the L2 every time.  So everything but
+// the tile itself is kept short: one form of the cursors for any number of sequences (in lanes, no shared memory), loops that
+// stay loops, and one merge by all threads instead of two rounds between warps (60 KB of instructions before, 33 now).  One 7B
+// sequence of 517 / 4000 tokens: 8.5 -> 7.5 / 12.9 -> 11.0 us with the merge of the pieces; 17 of 100 to 3000: 18.6 -> 16.9 us;
+// 14B, 64 of 128 to 2300: 69.6 -> 59.2 us cut, 57.1 -> 55.2 whole.
 template <int HD, bool EXT, int NB>
 __global__ void __launch_bounds__(kDecWarps * 32)
 attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restrict__ kv, const int* __restrict__ bt,
@@ -105,116 +112,85 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
   constexpr int kPitch = HD + 4;                       // floats per head in the merge buffers: conflict-free
   constexpr int kBuf = kHeads * kPitch + 2 * kHeads;   // O, then m and l per head
   extern __shared__ __align__(128) uint8_t smem[];
-  float* merge = reinterpret_cast<float*>(smem + kDecWarps * kDecStages * 2 * kTileBytes);
-  int* prefix = reinterpret_cast<int*>(merge + 3 * kBuf);      // [num_seqs + 1] tiles x nkv before a sequence
-  __shared__ int s_longest;
+  float* merge = reinterpret_cast<float*>(smem + kDecWarps * kDecStages * 2 * kTileBytes);      // a buffer per warp
   pdl_launch_dependents();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t2 = (lane & 3) * 2;
   const int G = nh / nkv;
-  // ---- lengths -> prefix sums of the tiles.  Up to 32 sequences stay in a warp's lanes (no barrier before the first load of
-  // keys); more go through shared memory.
-  const bool in_lanes = num_seqs <= 32;
-  int my_n = 0, my_incl = 0, longest = 0, total = 0;
-  if (in_lanes) {
-    my_n = lane < num_seqs ? seq_tiles(seq_lens[lane], EXT ? window : 0) : 0;
-    my_incl = my_n * nkv;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, my_incl, o);
-      if (lane >= o) my_incl += u;
-    }
-    longest = __reduce_max_sync(0xffffffffu, my_n);
-    total = __shfl_sync(0xffffffffu, my_incl, 31);
-  } else {
-    if (threadIdx.x == 0) s_longest = 0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < num_seqs; i += blockDim.x) {
-      const int n = seq_tiles(seq_lens[i], EXT ? window : 0);
-      prefix[i + 1] = n * nkv;
-      atomicMax(&s_longest, n);
-    }
-    __syncthreads();
-    if (warp == 0) {
-      int carry = 0;
-      for (int i = 0; i < num_seqs; i += 32) {
-        int v = i + lane < num_seqs ? prefix[i + lane + 1] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int u = __shfl_up_sync(0xffffffffu, v, o);
-          if (lane >= o) v += u;
-        }
-        if (i + lane < num_seqs) prefix[i + lane + 1] = carry + v;
-        carry += __shfl_sync(0xffffffffu, v, 31);
-      }
-      if (lane == 0) prefix[0] = 0;
-    }
-    __syncthreads();
-    longest = s_longest;
-    total = prefix[num_seqs];
-  }
-  auto tiles_of = [&](int i) {
-    return in_lanes ? __shfl_sync(0xffffffffu, my_n, i) : (prefix[i + 1] - prefix[i]) / nkv;
-  };
+  auto tiles_of = [&](int i) { return seq_tiles(seq_lens[i], EXT ? window : 0); };
   const bool whole = num_splits < 3;                   // items are not cut: CTA i has item i
-  const int per = whole ? 1 : tiles_per_cta(total, longest, gridDim.x, num_splits);
-  const int p_begin = whole ? int(blockIdx.x) : min(total, int(blockIdx.x) * per);
-  const int p_end = whole ? int(blockIdx.x) + 1 : min(total, p_begin + per);
+  int p_begin = blockIdx.x, p_end = p_begin + 1, per = 1;
+  if (!whole) {
+    int total = 0, longest = 0;
+    for (int i = lane; i < num_seqs; i += 32) {
+      const int n = tiles_of(i);
+      total += n * nkv;
+      longest = max(longest, n);
+    }
+    total = __reduce_add_sync(0xffffffffu, total);
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    per = tiles_per_cta(total, longest, gridDim.x, num_splits);
+    p_begin = min(total, int(blockIdx.x) * per);
+    p_end = min(total, p_begin + per);
+  }
 
+  // 32 neighbouring sequences in the lanes of a warp: tiles of sequence base + lane, and the position behind its last item.  No
+  // shared memory and no barriers; a cursor only moves forward.
+  struct Window {
+    int base, n, behind, end;
+  };
+  auto move_to = [&](Window& w, int p) {               // to the window that position p lies in
+    while (p >= w.end) {
+      w.base += 32;
+      w.n = w.base + lane < num_seqs ? tiles_of(w.base + lane) : 0;
+      w.behind = w.n * nkv;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, w.behind, o);
+        if (lane >= o) w.behind += u;
+      }
+      w.behind += w.end;
+      w.end = __shfl_sync(0xffffffffu, w.behind, 31);
+    }
+  };
   struct Seg {
     int seq, kvh, first, n, tiles;                     // tiles first .. first + n - 1 of `tiles` of the item
   };
   // the segment at position p (p < p_end), and the position behind it; the whole warp calls it
-  auto segment = [&](int p, Seg& sg) {
+  auto segment = [&](int p, Window& w, Seg& sg) {
     if (whole) {
       sg.seq = unsigned(p) / unsigned(nkv), sg.kvh = p - sg.seq * nkv;
       sg.first = 0;
       sg.tiles = sg.n = tiles_of(sg.seq);
       return p + 1;
     }
-    int begin;
-    if (in_lanes) {
-      sg.seq = __popc(__ballot_sync(0xffffffffu, my_incl <= p));
-      sg.tiles = __shfl_sync(0xffffffffu, my_n, sg.seq);
-      begin = __shfl_sync(0xffffffffu, my_incl, sg.seq) - sg.tiles * nkv;
-    } else {
-      int lo = 0, hi = num_seqs;
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (prefix[mid] <= p) lo = mid; else hi = mid;
-      }
-      sg.seq = lo;
-      sg.tiles = unsigned(prefix[lo + 1] - prefix[lo]) / unsigned(nkv);
-      begin = prefix[lo];
-    }
-    sg.kvh = unsigned(p - begin) / unsigned(sg.tiles);
-    sg.first = p - begin - sg.kvh * sg.tiles;
+    move_to(w, p);
+    const int at = __popc(__ballot_sync(0xffffffffu, w.behind <= p));
+    sg.seq = w.base + at;
+    sg.tiles = __shfl_sync(0xffffffffu, w.n, at);
+    const int in = p - (__shfl_sync(0xffffffffu, w.behind, at) - sg.tiles * nkv);
+    sg.kvh = unsigned(in) / unsigned(sg.tiles);
+    sg.first = in - sg.kvh * sg.tiles;
     sg.n = min(sg.tiles - sg.first, p_end - p);
     return p + sg.n;
   };
 
   // ---- this warp's tiles, one after the other over all segments: what is fetched next
   uint8_t* ring = smem + warp * (kDecStages * 2 * kTileBytes);
+  Window fw{-32, 0, 0, 0};
+  if (p_begin < p_end && !whole) move_to(fw, p_begin);
+  Window cw = fw;
   Seg fs{};
   int fp = p_begin, fi = 0, f_tile0 = 0;
-  bool f_live = true;
-  fs.n = 0;
-  auto f_seek = [&]() {                                // fi past the end of the segment: on to one with a tile for this warp
-    while (fi >= fs.n) {
-      if (fp >= p_end) {
-        f_live = false;
-        return;
-      }
-      fp = segment(fp, fs);
+  uint32_t holes = 0;                                  // bit = ring slot whose tile lies in a dropped block
+  auto issue = [&](int slot) {                         // next tile -> ring slot; always commits a group
+    while (fi >= fs.n && fp < p_end) {                 // on to a segment with a tile for this warp
+      fp = segment(fp, fw, fs);
       fi = warp;
       f_tile0 = (EXT && window > 0 ? max(0, seq_lens[fs.seq] - window) >> 4 : 0) + fs.first;
     }
-  };
-  f_seek();
-  uint32_t holes = 0;                                  // bit = ring slot whose tile lies in a dropped block
-  auto issue = [&](int slot) {                         // next tile -> ring slot; always commits a group
     holes &= ~(1u << slot);
-    if (f_live) {
+    if (fi < fs.n) {
       const int tile = f_tile0 + fi;
       const int bi = block_shift >= 0 ? tile >> block_shift : tile / (block_size >> 4);
       const int in = tile - bi * (block_size >> 4);
@@ -234,24 +210,17 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
         holes |= 1u << slot;
       }
       fi += kDecWarps;
-      f_seek();
     }
     cp_async_commit();
   };
-#pragma unroll
+#pragma unroll 1
   for (int i = 0; i < kDecStages - 1; ++i) issue(i);
 
-  for (int i = blockIdx.x; i < num_seqs; i += gridDim.x)       // sequences of nothing: zeros
-    if (tiles_of(i) == 0) {
-      for (int d = threadIdx.x; d < nh * HD; d += blockDim.x) out[size_t(i) * ldo + d] = __float2half_rn(0.f);
-      if (!whole)
-        for (int h = threadIdx.x; h < nh; h += blockDim.x) *piece_count(scratch, i * nh + h, num_splits, HD) = 1;
-    }
   int slot = 0;
   for (int p = p_begin; p < p_end;) {
     Seg sg;
     const int here = p;
-    p = segment(p, sg);
+    p = segment(p, cw, sg);
     if (sg.n == 0) continue;                           // (a whole item: an empty sequence)
     const int len = seq_lens[sg.seq];
     const int first_tok = EXT && window > 0 ? max(0, len - window) : 0;
@@ -345,92 +314,75 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
         for (int nb = 0; nb < NB; ++nb) mma16816(o[nb][d], a, pb[nb][0], pb[nb][1]);
       }
     }
-    // ---- merge the four warps: 2 and 3 into 0 and 1, 1 into 0.  (Three buffers: nobody writes one that may still be read.)
+    // ---- the four warps give what they have, all threads add it up
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
       for (int e = 0; e < 2; ++e)
 #pragma unroll
         for (int sh = 4; sh < 32; sh <<= 1) l[nb][e] += __shfl_xor_sync(0xffffffffu, l[nb][e], sh);
-    auto give = [&](float* buf) {
+    __syncthreads();                                   // (the item before has been read)
+    float* mine = merge + warp * kBuf;
 #pragma unroll
-      for (int nb = 0; nb < NB; ++nb)
+    for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int h = nb * 8 + t2 + e;
+      for (int e = 0; e < 2; ++e) {
+        const int h = nb * 8 + t2 + e;
 #pragma unroll
-          for (int d = 0; d < kSteps; ++d) {
-            buf[h * kPitch + d * 16 + g] = o[nb][d][e];
-            buf[h * kPitch + d * 16 + g + 8] = o[nb][d][2 + e];
-          }
-          if (g == 0) {
-            buf[kHeads * kPitch + h] = m[nb][e];
-            buf[kHeads * kPitch + kHeads + h] = l[nb][e];
-          }
+        for (int d = 0; d < kSteps; ++d) {
+          mine[h * kPitch + d * 16 + g] = o[nb][d][e];
+          mine[h * kPitch + d * 16 + g + 8] = o[nb][d][2 + e];
         }
-    };
-    auto take = [&](const float* buf) {
-#pragma unroll
-      for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int h = nb * 8 + t2 + e;
-          const float om = buf[kHeads * kPitch + h], n = fmaxf(m[nb][e], om);
-          const float fa = m[nb][e] == -INFINITY ? 0.f : ex2_approx(m[nb][e] - n);
-          const float fb = om == -INFINITY ? 0.f : ex2_approx(om - n);
-          m[nb][e] = n;
-          l[nb][e] = l[nb][e] * fa + buf[kHeads * kPitch + kHeads + h] * fb;
-#pragma unroll
-          for (int d = 0; d < kSteps; ++d) {
-            o[nb][d][e] = o[nb][d][e] * fa + buf[h * kPitch + d * 16 + g] * fb;
-            o[nb][d][2 + e] = o[nb][d][2 + e] * fa + buf[h * kPitch + d * 16 + g + 8] * fb;
-          }
+        if (g == 0) {
+          mine[kHeads * kPitch + h] = m[nb][e];
+          mine[kHeads * kPitch + kHeads + h] = l[nb][e];
         }
-    };
-    if (warp >= 2) give(merge + (warp - 2) * kBuf);
+      }
     __syncthreads();
-    if (warp < 2) take(merge + warp * kBuf);
-    if (warp == 1) give(merge + 2 * kBuf);
-    __syncthreads();
-    if (warp == 0) {
-      take(merge + 2 * kBuf);
-      const int start = whole ? 0 : here - sg.first;             // position of the item's first tile
-      const int pieces = whole ? 1 : (start + sg.tiles - 1) / per - start / per + 1;
-      const bool alone = pieces == 1;
-      const int piece = alone ? 0 : int(blockIdx.x) - start / per;
-      if (!whole && sg.first == 0 && lane < G) *piece_count(scratch, sg.seq * nh + sg.kvh * G + lane, num_splits, HD) = pieces;
+    const int start = whole ? 0 : here - sg.first;               // position of the item's first tile
+    const int pieces = whole ? 1 : (start + sg.tiles - 1) / per - start / per + 1;
+    const bool alone = pieces == 1;
+    const int piece = alone ? 0 : int(blockIdx.x) - start / per;
+    if (!whole && sg.first == 0 && threadIdx.x < G)
+      *piece_count(scratch, sg.seq * nh + sg.kvh * G + threadIdx.x, num_splits, HD) = pieces;
+    constexpr int kPart = HD / 4;                                // a thread: four elements this far apart
+#pragma unroll 1
+    for (int idx = threadIdx.x; idx < G * kPart; idx += kDecWarps * 32) {
+      const int h = idx / kPart, d = idx % kPart, head = sg.kvh * G + h;
+      float mw[kDecWarps], M = -INFINITY, L = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int nb = 0; nb < NB; ++nb)
+      for (int w = 0; w < kDecWarps; ++w) M = fmaxf(M, mw[w] = merge[w * kBuf + kHeads * kPitch + h]);
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int h = nb * 8 + t2 + e;
-          if (h < G) {
-            const int head = sg.kvh * G + h;
-            if (alone) {
-              __half* dst = out + size_t(sg.seq) * ldo + size_t(head) * HD + g;
-              const float inv = l[nb][e] > 0.f ? 1.f / l[nb][e] : 0.f;
+      for (int w = 0; w < kDecWarps; ++w) {
+        const float* src = merge + w * kBuf;
+        const float f = mw[w] == -INFINITY ? 0.f : ex2_approx(mw[w] - M);
+        L += src[kHeads * kPitch + kHeads + h] * f;
 #pragma unroll
-              for (int d = 0; d < kSteps; ++d) {
-                dst[d * 16] = __float2half_rn(o[nb][d][e] * inv);
-                dst[d * 16 + 8] = __float2half_rn(o[nb][d][2 + e] * inv);
-              }
-            } else {
-              float* dst = scratch + (size_t(sg.seq * nh + head) * num_splits + piece) * (HD + 2);
+        for (int k = 0; k < 4; ++k) acc[k] += src[h * kPitch + d + k * kPart] * f;
+      }
+      if (alone) {
+        __half* dst = out + size_t(sg.seq) * ldo + size_t(head) * HD + d;
+        const float inv = L > 0.f ? 1.f / L : 0.f;
 #pragma unroll
-              for (int d = 0; d < kSteps; ++d) {
-                dst[d * 16 + g] = o[nb][d][e];
-                dst[d * 16 + g + 8] = o[nb][d][2 + e];
-              }
-              if (g == 0) {
-                dst[HD] = m[nb][e];
-                dst[HD + 1] = l[nb][e];
-              }
-            }
-          }
+        for (int k = 0; k < 4; ++k) dst[k * kPart] = __float2half_rn(L > 0.f ? acc[k] * inv : 0.f);
+      } else {
+        float* dst = scratch + (size_t(sg.seq * nh + head) * num_splits + piece) * (HD + 2);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) dst[d + k * kPart] = acc[k];
+        if (d == 0) {
+          dst[HD] = M;
+          dst[HD + 1] = L;
         }
+      }
     }
   }
   cp_async_wait<0>();
+  for (int i = blockIdx.x; i < num_seqs; i += gridDim.x)         // sequences of nothing: zeros
+    if (tiles_of(i) == 0) {
+      for (int d = threadIdx.x; d < nh * HD; d += blockDim.x) out[size_t(i) * ldo + d] = __float2half_rn(0.f);
+      if (!whole)
+        for (int h = threadIdx.x; h < nh; h += blockDim.x) *piece_count(scratch, i * nh + h, num_splits, HD) = 1;
+    }
 }
 
 // Items that attn_decode_kernel cut in pieces.  grid (nh, sequences), HD threads.
@@ -440,22 +392,44 @@ __global__ void attn_combine_kernel(float* __restrict__ scratch, __half* __restr
   pdl_wait();
   const int head = blockIdx.x, seq = blockIdx.y, d = threadIdx.x;
   const float* src = scratch + size_t(seq * nh + head) * num_splits * (HD + 2);
-  // the records are read beside the count (num_splits >= 3: two are there, whatever they hold), not behind it
+  // what a few pieces need is read beside their number, not behind it (num_splits >= 3: places that exist, whatever they hold);
+  // lane s has the maximum and the sum of piece s
+  const int lane = threadIdx.x & 31, some = num_splits - 1;
   const int pieces = *piece_count(scratch, seq * nh + head, num_splits, HD);
-  const float m0 = src[HD], l0 = src[HD + 1], o0 = src[d], m1 = src[2 * HD + 2], l1 = src[2 * HD + 3], o1 = src[HD + 2 + d];
+  float m = lane < some ? src[lane * (HD + 2) + HD] : -INFINITY, l = lane < some ? src[lane * (HD + 2) + HD + 1] : 0.f;
+  float o[4];
+#pragma unroll
+  for (int s = 0; s < 4; ++s) o[s] = s < some ? src[s * (HD + 2) + d] : 0.f;
   if (pieces == 1) return;                             // its CTA stored it
-  float M = fmaxf(m0, m1);
-  for (int s = 2; s < pieces; ++s) M = fmaxf(M, src[s * (HD + 2) + HD]);
-  const float f0 = m0 == -INFINITY ? 0.f : ex2_approx(m0 - M), f1 = m1 == -INFINITY ? 0.f : ex2_approx(m1 - M);
-  float L = l0 * f0 + l1 * f1, acc = o0 * f0 + o1 * f1;
-#pragma unroll 4
-  for (int s = 2; s < pieces; ++s) {
-    const float ms = src[s * (HD + 2) + HD];
-    const float f = ms == -INFINITY ? 0.f : ex2_approx(ms - M);
-    L += src[s * (HD + 2) + HD + 1] * f;
-    acc += src[s * (HD + 2) + d] * f;
+  __half* dst = out + size_t(seq) * ldo + size_t(head) * HD + d;
+  if (pieces > 32) {
+    float M = -INFINITY, L = 0.f, acc = 0.f;
+    for (int s = 0; s < pieces; ++s) M = fmaxf(M, src[s * (HD + 2) + HD]);
+    for (int s = 0; s < pieces; ++s) {
+      const float ms = src[s * (HD + 2) + HD], f = ms == -INFINITY ? 0.f : ex2_approx(ms - M);
+      L += src[s * (HD + 2) + HD + 1] * f;
+      acc += src[s * (HD + 2) + d] * f;
+    }
+    *dst = __float2half_rn(L > 0.f ? acc / L : 0.f);
+    return;
   }
-  out[size_t(seq) * ldo + size_t(head) * HD + d] = __float2half_rn(L > 0.f ? acc / L : 0.f);
+  m = lane < pieces ? m : -INFINITY;
+  float M = m;
+#pragma unroll
+  for (int sh = 16; sh > 0; sh >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, sh));
+  const float f = m == -INFINITY ? 0.f : ex2_approx(m - M);
+  float L = lane < pieces ? l * f : 0.f;
+#pragma unroll
+  for (int sh = 16; sh > 0; sh >>= 1) L += __shfl_xor_sync(0xffffffffu, L, sh);
+  float acc = 0.f;
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const float fs = __shfl_sync(0xffffffffu, f, s);
+    if (s < pieces) acc += o[s] * fs;
+  }
+#pragma unroll 4
+  for (int s = 4; s < pieces; ++s) acc += src[s * (HD + 2) + d] * __shfl_sync(0xffffffffu, f, s);
+  *dst = __float2half_rn(L > 0.f ? acc / L : 0.f);
 }
 
 // ---- prefill / chunked prefill / verify ----------------------------------------------------------------
@@ -647,12 +621,9 @@ extern "C" int64_t zse_attn_decode_scratch_floats(int num_seqs, int nh, int hd, 
   return int64_t(num_seqs) * nh * max_splits * (hd + 2);
 }
 
-// Shared memory of the decode kernel: rings, three merge buffers, prefix sums of the lengths.
+// Shared memory of the decode kernel: rings and a merge buffer per warp.
 template <int HD, int NB>
-constexpr int decode_smem(int num_seqs) {
-  return kDecWarps * kDecodeStages<HD, NB> * 2 * 16 * HD * 2 + 3 * (8 * NB * (HD + 4) + 2 * 8 * NB) * 4 + (num_seqs + 1) * 4;
-}
-constexpr int kDecMaxSeqs = 2048;                        // sequences of one call, bounded by the prefix sums' place
+constexpr int kDecodeSmem = kDecWarps * (kDecodeStages<HD, NB> * 2 * 16 * HD * 2 + (8 * NB * (HD + 4) + 2 * 8 * NB) * 4);
 
 // The attribute is raised once per device (host work: not a stream operation).
 template <int HD, bool EXT, int NB>
@@ -661,7 +632,7 @@ static int prepare_decode() {
   const int dev_slot = current_device_slot();
   if (!attr[dev_slot]) {
     if (cudaFuncSetAttribute(attn_decode_kernel<HD, EXT, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             decode_smem<HD, NB>(kDecMaxSeqs)) != cudaSuccess)
+                             kDecodeSmem<HD, NB>) != cudaSuccess)
       return ZSE_ERR_LAUNCH;
     attr[dev_slot] = true;
   }
@@ -690,23 +661,18 @@ static int launch_decode(const void* q, int ldq, const void* kv, const void* bt,
   while ((1 << shift) < tpb) ++shift;
   if ((1 << shift) != tpb) shift = -1;
   // cut: as many CTAs as the chip holds at once (rings of 48, 96 and 192 KB), each with the same share of the tiles
-  for (int s0 = 0; s0 < num_seqs; s0 += kDecMaxSeqs) {   // (one round in practice)
-    const int n = min(kDecMaxSeqs, num_seqs - s0);
-    const int fit = decode_sms() * (HD == 256 ? 1 : HD == 128 ? 2 : 4);
-    const int ctas = splits >= 3 ? min(fit, n * nkv * (splits - 1)) : n * nkv;         // (with few sequences most of the chip is left to the next kernel)
-    const __half* q0 = reinterpret_cast<const __half*>(q) + size_t(s0) * ldq;
-    __half* o0 = reinterpret_cast<__half*>(out) + size_t(s0) * ldo;
-    const int *bt0 = reinterpret_cast<const int*>(bt) + size_t(s0) * max_blocks, *l0 = reinterpret_cast<const int*>(lens) + s0;
-    if (launch_pdl(attn_decode_kernel<HD, EXT, NB>, dim3(ctas), dim3(kDecWarps * 32), size_t(decode_smem<HD, NB>(n)), st, q0,
-                   ldq, reinterpret_cast<const __half*>(kv), bt0, max_blocks, l0, o0, ldo, reinterpret_cast<float*>(scratch), n,
-                   nh, nkv, block_size, shift, splits, scale * kLog2e, blk_stride, half_stride, softcap,
-                   window) != cudaSuccess)
+  const int fit = decode_sms() * (HD == 256 ? 1 : HD == 128 ? 2 : 4);
+  const int ctas = splits >= 3 ? min(fit, num_seqs * nkv * (splits - 1)) : num_seqs * nkv;   // (with few sequences most of the chip is left to the next kernel)
+  if (launch_pdl(attn_decode_kernel<HD, EXT, NB>, dim3(ctas), dim3(kDecWarps * 32), size_t(kDecodeSmem<HD, NB>), st,
+                 reinterpret_cast<const __half*>(q), ldq, reinterpret_cast<const __half*>(kv), reinterpret_cast<const int*>(bt),
+                 max_blocks, reinterpret_cast<const int*>(lens), reinterpret_cast<__half*>(out), ldo,
+                 reinterpret_cast<float*>(scratch), num_seqs, nh, nkv, block_size, shift, splits, scale * kLog2e, blk_stride,
+                 half_stride, softcap, window) != cudaSuccess)
+    return ZSE_ERR_LAUNCH;
+  if (splits >= 3) {
+    if (launch_pdl(attn_combine_kernel<HD>, dim3(nh, num_seqs), dim3(HD), 0, st, reinterpret_cast<float*>(scratch),
+                   reinterpret_cast<__half*>(out), ldo, nh, splits) != cudaSuccess)
       return ZSE_ERR_LAUNCH;
-    if (splits >= 3) {
-      if (launch_pdl(attn_combine_kernel<HD>, dim3(nh, n), dim3(HD), 0, st, reinterpret_cast<float*>(scratch), o0, ldo, nh,
-                     splits) != cudaSuccess)
-        return ZSE_ERR_LAUNCH;
-    }
   }
   return 0;
 }

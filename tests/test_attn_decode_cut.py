@@ -77,3 +77,11 @@ def test_decode_attention(hd, nh, nkv, bs, softcap, window, splits, lens):
     # probabilities and the result in fp16 (2^-11 each), keys and values exact
     assert float((out.double() - want).norm() / want.norm()) < 1.2e-3
     assert (out[ln == 0] == 0).all() and torch.isfinite(out).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("splits,lens", [(64, [4096, 30]), (33, [9000]), (34, [9000, 1]), (16, [(7 * i) % 90 for i in range(300)]),
+                                         (5, [900] + [0] * 2100 + [50])])
+def test_many_pieces_and_many_sequences(splits, lens):
+    """More pieces than a warp has lanes, more sequences than one window of 32, sequences of nothing in between."""
+    test_decode_attention(128, 8, 2, 16, 0, 0, splits, lens)
