@@ -333,8 +333,23 @@ int gemm_w4_small_planes(int N, int K, int want_split) {
 
 bool gemm_w4_small_takes(int M, int K) { return M >= 1 && M <= 8 && K > 0 && K % kW4StageK == 0; }
 
+// These CTAs start while the attention kernel and others with most of an SM's shared memory still run, and fetch their weights
+// meanwhile.  That needs an SM whose split between shared memory and L1 suits both: left to the driver's choice the launch waits
+// until SMs are empty.  Anything from 25 to 75 % avoids it (100 % does not), and the L1 serves the activations of 8 tokens: 7168 x 14336,
+// fp16, 16.3 us at 25 % and 17.1 at 50.  7B steps, driver's choice -> 25 %: one sequence of 517 tokens 1820 -> 1710 us, of 4000
+// 1950 -> 1808, 8 of 517 2090 -> 1872.
+constexpr int kSmallCarveout = 25;
+
 template <int EPI>
 static int launch_small(const SmallArgs& a, cudaStream_t st) {
+  static bool attr_done[kMaxDevices] = {};
+  const int dev = current_device_slot();
+  if (!attr_done[dev]) {
+    if (cudaFuncSetAttribute(gemm_w4_small_kernel<EPI>, cudaFuncAttributePreferredSharedMemoryCarveout, kSmallCarveout) !=
+        cudaSuccess)
+      return ZSE_ERR_LAUNCH;
+    attr_done[dev] = true;
+  }
   const int sms = small_sms();
   const bool two = a.items > sms;
   const int threads = two ? kSmallThreads / 2 : kSmallThreads;
