@@ -48,6 +48,8 @@ int zse_gemm_w4_dec_qkv_rope(const void* w_tiled, const void* x, int x_rows_cap,
                              int max_position, void* workspace, void* status, void* stream);
 // the plan of a call: out2 = {CTAs, K segments per tile pair (0: the stream plan)}
 void zse_gemm_w4_dec_plan(int N, int K, int epilogue, int sm_count, int* out2);
+// 1 when an INT4 call of these sizes (epilogue 3: fused QKV) runs in gemm_w4_small.cu
+int zse_gemm_w4_dec_small(int M, int N, int K, int epilogue);
 void zse_gemm_w4_dec_set_tuning(int min_steps, int max_split);
 
 int zse_gemm_f16(const void* w, int w_rows_cap, const void* x, int x_rows_cap, const void* bias, void* out, int M,

@@ -92,6 +92,8 @@ struct GatherWait {
 };
 int tp_fill_sp_table(const void* ctx, int slot, bool multimem, int rank_override, SpTable* out);
 
+extern int g_w4_mode;          // tuning hook, see gemm_w4.cu
+
 // Up to 8 tokens on INT4 chunks (gemm_w4_small.cu); epilogues fp16, SwiGLU, fp32 planes and kEpiQkvRope (N = (nh + 2 nkv) * 128).
 // gemm_w4_small_planes: planes the third writes.
 struct SmallRope {
@@ -101,7 +103,8 @@ struct SmallRope {
   __half* kv_layer;            // [blocks][2][nkv][block_size][128]
   int nh, nkv, block_size, max_position;
 };
-bool gemm_w4_small_takes(int M, int K);
+// The rule for who takes a call: split_plan = the other candidate is gemm_w4_dec.cu, otherwise gemm_w4.cu.
+bool gemm_w4_small_takes(int M, int N, int K, int epilogue, bool split_plan);
 int gemm_w4_small_planes(int N, int K, int want_split);
 int gemm_w4_small_run(const void* w_tiled, const void* x, const void* bias, void* out, int M, int N, int K, int ldo,
                       int epilogue, int want_split, const SmallRope* rope, cudaStream_t st);

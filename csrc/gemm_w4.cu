@@ -845,7 +845,7 @@ static int launch_w4_epi(int epilogue, const CUtensorMap& tx, const W4Args& a, d
 
 // 0 = the planner decides, 1 = wide CTAs only, 2 = narrow (two per SM) CTAs wherever they are allowed;
 // adding 4 keeps calls of up to 8 tokens on the kernels of this file instead of gemm_w4_small.cu
-static int g_w4_mode = 0;
+int g_w4_mode = 0;
 
 // How the launcher tiles a problem: weight tiles per CTA (R) and K splits (ks).  Measured on B200: a tcgen05.mma of
 // M=128, K=16 occupies the tensor pipe for about 50 cycles whatever N <= 64 is, so a 128x128 weight chunk costs about
@@ -925,11 +925,12 @@ extern "C" void zse_gemm_w4_set_timing(void* dev_buffer) { g_w4_timing = reinter
 // Tuning hook: 0 = planner decides between wide and narrow CTAs, 1 = wide only, 2 = narrow wherever allowed.
 extern "C" void zse_gemm_w4_set_mode(int mode) { zse::g_w4_mode = mode; }
 
-// Up to 8 tokens: gemm_w4_small.cu, unless a tuning mode or a cluster along K asks for a CTA of this file.  Measured (B200, cold
+// Up to 8 tokens: gemm_w4_small.cu, unless a tuning mode or a cluster along K asks for a CTA of this file or the layer is narrow
+// and deep (gemm_w4_small_takes).  Measured (B200, cold
 // L2, this file -> that one), 5 tokens: 7B gate/up 32.8 -> 23.5 us, down 21.5 -> 16.4, QKV 16.4 -> 12.3; a variant for 16 tokens
 // lost (gate/up 32.8 -> 41.8 us: twice the products, fewer warps for its registers).
-static bool takes_small(int M, int K, int epilogue, int k_split) {
-  return g_w4_mode == 0 && gemm_w4_small_takes(M, K) && (epilogue == kEpiPartialF32 || k_split <= 0);
+static bool takes_small(int M, int N, int K, int epilogue, int k_split) {
+  return (epilogue == kEpiPartialF32 || k_split <= 0) && gemm_w4_small_takes(M, N, K, epilogue, false);
 }
 
 // More than 64 tokens: gemm_pair.cu, except for narrow layers whose epilogue needs the whole sum.  They leave most pairs without
@@ -955,7 +956,7 @@ static int run_gemm_w4(const void* w_tiled, const void* x, int x_rows_cap, const
     if (sm_count <= 0) sm_count = 148;
   }
   if ((sp != nullptr || gather != nullptr) && M <= 64) return ZSE_ERR_SHAPE;   // wide CTAs (128 / 256 tokens) only
-  if (push == nullptr && takes_small(M, K, epilogue, k_split))
+  if (push == nullptr && takes_small(M, N, K, epilogue, k_split))
     return gemm_w4_small_run(w_tiled, x, bias, out, M, N, K, ldo, epilogue, k_split, nullptr,
                              reinterpret_cast<cudaStream_t>(stream));
   if (push == nullptr && sp == nullptr && takes_pair(M, N, epilogue, sm_count))
@@ -1085,7 +1086,7 @@ extern "C" int zse_gemm_w4_max_clusters(int narrow, int cluster) {
 // CTA shape (0 wide, 1 narrow)}; -1 in out4[3] = gemm_w4_small.cu.
 extern "C" void zse_gemm_w4_plan(int M, int N, int K, int epilogue, int k_split, int sm_count, int* out4) {
   if (sm_count <= 0) sm_count = 148;
-  if (takes_small(M, K, epilogue, k_split)) {
+  if (takes_small(M, N, K, epilogue, k_split)) {
     out4[0] = 1, out4[1] = epilogue == kEpiPartialF32 ? gemm_w4_small_planes(N, K, k_split) : 1, out4[2] = 1, out4[3] = -1;
     return;
   }
@@ -1099,7 +1100,7 @@ extern "C" int zse_gemm_w4_splits(int M, int N, int K, int k_split) {
   int sm_count = 148, dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
   if (sm_count <= 0) sm_count = 148;
-  if (takes_small(M, K, kEpiPartialF32, k_split)) return gemm_w4_small_planes(N, K, k_split);
+  if (takes_small(M, N, K, kEpiPartialF32, k_split)) return gemm_w4_small_planes(N, K, k_split);
   if (M > 64) return gemm_pair_planes(M, N, K, k_split);
   int R = 1, ks = 1, cluster = 1, dual = 0;
   plan_w4(M, N, K, kEpiPartialF32, sm_count, k_split, &R, &ks, &cluster, &dual);

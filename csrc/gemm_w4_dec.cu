@@ -1405,6 +1405,15 @@ extern "C" int zse_gemm_w4_dec_supported(int M, int N, int K, int epilogue) {
   return (epilogue == kDecF16 || epilogue == kDecF32) && (N % 8) == 0 ? 1 : 0;
 }
 
+static int small_epilogue(int epilogue) {
+  return epilogue == kDecF16 ? kEpiF16 : epilogue == kDecSwiGLU ? kEpiSwiGLU : epilogue == kDecF32 ? kEpiPartialF32 : kEpiQkvRope;
+}
+
+// 1 when an INT4 call with these sizes runs in gemm_w4_small.cu
+extern "C" int zse_gemm_w4_dec_small(int M, int N, int K, int epilogue) {
+  return epilogue != kDecAllReduceNorm && gemm_w4_small_takes(M, N, K, small_epilogue(epilogue), true) ? 1 : 0;
+}
+
 static int run_dec(bool w8, const void* w_tiled, const void* x, int x_rows_cap, const void* bias, void* out, int M,
                    int N, int K, int ldo, int epilogue, void* workspace, const DecRope* rope, void* status,
                    void* stream, const DecTpNorm* tpn = nullptr) {
@@ -1414,9 +1423,8 @@ static int run_dec(bool w8, const void* w_tiled, const void* x, int x_rows_cap, 
       (reinterpret_cast<uintptr_t>(bias) & 15))
     return ZSE_ERR_ALIGN;
   if (epilogue == kDecF32 ? (ldo % 4) : (ldo % 8)) return ZSE_ERR_ALIGN;
-  if (!w8 && epilogue != kDecAllReduceNorm && gemm_w4_small_takes(M, K)) {
-    const int epi = epilogue == kDecF16 ? kEpiF16 : epilogue == kDecSwiGLU ? kEpiSwiGLU
-                    : epilogue == kDecF32 ? kEpiPartialF32 : kEpiQkvRope;
+  if (!w8 && zse_gemm_w4_dec_small(M, N, K, epilogue)) {
+    const int epi = small_epilogue(epilogue);
     SmallRope sr{};
     if (rope != nullptr)
       sr = SmallRope{rope->positions, rope->slots, rope->cos_sin, rope->kv_layer, rope->nh, rope->nkv, rope->block_size,

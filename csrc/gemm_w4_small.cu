@@ -331,7 +331,18 @@ int gemm_w4_small_planes(int N, int K, int want_split) {
   return (k_stages + spp - 1) / spp;                           // no empty split
 }
 
-bool gemm_w4_small_takes(int M, int K) { return M >= 1 && M <= 8 && K > 0 && K % kW4StageK == 0; }
+// Epilogues that need the whole sum have no K splits here, so the time of a narrow layer goes with its depth alone (1.7 us and 0.9 a
+// thousand columns), while a cluster along K (gemm_w4.cu) or the split plan of gemm_w4_dec.cu has more CTAs for it.  Measured (B200,
+// weights from memory, 4 tokens; here | cluster | split plan, us): 8 tiles of 4096: 5.5 | 6.2 | 6.0, of 8192: 9.0 | 7.9 | 8.6;
+// 16 of 5632: 7.3 | 7.6 | 8.2, of 8192: 9.0 | 8.6 | 9.5, of 16384: 16.0 | 12.7 | 15.1; 28 of 4096 (Gemma-2 9B o_proj): 5.7 | 7.5 | 7.8, of
+// 10240: 11.1 | 11.2 | 11.9, of 14336 (down_proj): 14.6 | 13.4 | 14.7; 32 of 14336: 14.6 | 14.1 | 17.5; 36 of 21504: 20.9 | 28 | 24; 40
+// of 13824: 14.5 | 19.2 | 17.4.  More than 32 tiles have no room for clusters of eight at once.
+bool gemm_w4_small_takes(int M, int N, int K, int epilogue, bool split_plan) {
+  if (g_w4_mode != 0 || M < 1 || M > 8 || K <= 0 || K % kW4StageK != 0) return false;
+  if (epilogue == kEpiPartialF32) return true;
+  const int tiles = small_tiles(N, epilogue), k_stages = K / kW4StageK;
+  return split_plan ? tiles > 28 || k_stages <= 33 + 3 * tiles : tiles > 32 || k_stages * (57 - tiles) <= 2400;
+}
 
 // These CTAs start while the attention kernel and others with most of an SM's shared memory still run, and fetch their weights
 // meanwhile.  That needs an SM whose split between shared memory and L1 suits both: left to the driver's choice the launch waits
@@ -361,7 +372,7 @@ static int launch_small(const SmallArgs& a, cudaStream_t st) {
 
 int gemm_w4_small_run(const void* w_tiled, const void* x, const void* bias, void* out, int M, int N, int K, int ldo,
                       int epilogue, int want_split, const SmallRope* rope, cudaStream_t st) {
-  if (!gemm_w4_small_takes(M, K) || N <= 0) return ZSE_ERR_SHAPE;
+  if (M < 1 || M > 8 || K <= 0 || K % kW4StageK != 0 || N <= 0) return ZSE_ERR_SHAPE;
   if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w_tiled) & 15)) return ZSE_ERR_ALIGN;
   const int k_stages = K / kW4StageK, n_half = 2 * small_tiles(N, epilogue);
   const int ks = epilogue == kEpiPartialF32 ? gemm_w4_small_planes(N, K, want_split) : 1;

@@ -134,6 +134,8 @@ _SIGS = {
     "zse_gemm_w4_dec_workspace_bytes": (c_int64, [c_int]),
     "zse_gemm_w4_dec_supported": (c_int, [c_int, c_int, c_int, c_int]),
     "zse_gemm_w4_dec_plan": (None, [c_int, c_int, c_int, c_int, POINTER(c_int)]),
+    "zse_gemm_w4_dec_small": (c_int, [c_int, c_int, c_int, c_int]),
+    "zse_gemm_w4_plan": (None, [c_int, c_int, c_int, c_int, c_int, c_int, POINTER(c_int)]),
     "zse_gemm_w4_dec_set_tuning": (None, [c_int, c_int]),
     "zse_gemm_f16": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                              c_int, c_void_p, c_void_p]),
@@ -432,6 +434,19 @@ def gemm_w4_dec_plan(N, K, epilogue, sm_count):
     out = (c_int * 2)()
     load().zse_gemm_w4_dec_plan(N, K, epilogue, sm_count, out)
     return out[0], out[1]
+
+
+def gemm_w4_dec_small(M, N, K, epilogue) -> bool:
+    """Whether ``gemm_w4_dec`` (epilogue 3: ``gemm_w4_dec_qkv_rope``) runs such a call in csrc/gemm_w4_small.cu."""
+    return bool(load().zse_gemm_w4_dec_small(M, N, K, epilogue))
+
+
+def gemm_w4_plan(M, N, K, epilogue, k_split=0, sm_count=148):
+    """What ``gemm_w4`` does for a call: (tiles per wide CTA, K splits, cluster size, kind: 0 wide CTAs, 1 narrow CTAs, -1
+    csrc/gemm_w4_small.cu)."""
+    out = (c_int * 4)()
+    load().zse_gemm_w4_plan(M, N, K, epilogue, k_split, sm_count, out)
+    return tuple(out)
 
 
 def gemm_f16(w, w_rows, x, x_rows_cap, bias, out, M, N, K, ldo, epilogue, k_split, status):
