@@ -380,6 +380,8 @@ int zse_norm_add_rmsnorm(const void* x_f16, const void* w_post, void* residual_f
 int zse_softcap_f16(void* x_f16, int ld, int M, int V, float cap, void* stream);
 
 // ---- attention.cu -------------------------------------------------------------------------------------------
+// num_splits of decode attention: 1 = a CTA per (sequence, kv head); 2 = two, half the tokens each; N >= 3 = equal shares of all
+// tokens for every CTA, a (sequence, kv head) in at most N - 1 pieces.  Above 1 scratch is needed.
 int64_t zse_attn_decode_scratch_floats(int num_seqs, int nh, int hd, int max_splits);
 int zse_attn_decode(const void* q, int ldq, const void* kv_layer, const void* block_tables_i32, int max_blocks,
                     const void* seq_lens_i32, void* out_f16, int ldo, void* scratch_f32, int num_seqs, int nh, int nkv,

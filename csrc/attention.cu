@@ -61,7 +61,8 @@ __device__ __forceinline__ uint32_t tile_off(int row, int chunk) {
 // All 16-token tiles of all (sequence, kv head) items stand in one line, sequence by sequence.  With num_splits > 1 every CTA
 // takes the same number of them, `per`, whatever items they belong to; an item that lies in several CTAs is merged from scratch
 // by attn_combine_kernel (at most num_splits - 1 pieces: `per` is raised for that if one sequence is very long).  The last of a
-// head's num_splits records in scratch says how many pieces there are.  With num_splits < 3 items stay whole.
+// head's num_splits records in scratch says how many pieces there are.  That leaves nothing for two pieces, so with num_splits = 2
+// every item is cut in two halves; with 1 items stay whole.
 template <int HD, int NB>
 constexpr int kDecodeStages = HD == 256 && NB == 2 ? 2 : 3;       // of a warp's ring
 __device__ __forceinline__ int seq_tiles(int len, int window) {
@@ -118,9 +119,9 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t2 = (lane & 3) * 2;
   const int G = nh / nkv;
   auto tiles_of = [&](int i) { return seq_tiles(seq_lens[i], EXT ? window : 0); };
-  const bool whole = num_splits < 3;                   // items are not cut: CTA i has item i
+  const bool fixed = num_splits < 3;                   // CTA i has item i, or one half of item i / 2
   int p_begin = blockIdx.x, p_end = p_begin + 1, per = 1;
-  if (!whole) {
+  if (!fixed) {
     int total = 0, longest = 0;
     for (int i = lane; i < num_seqs; i += 32) {
       const int n = tiles_of(i);
@@ -158,10 +159,13 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
   };
   // the segment at position p (p < p_end), and the position behind it; the whole warp calls it
   auto segment = [&](int p, Window& w, Seg& sg) {
-    if (whole) {
-      sg.seq = unsigned(p) / unsigned(nkv), sg.kvh = p - sg.seq * nkv;
-      sg.first = 0;
-      sg.tiles = sg.n = tiles_of(sg.seq);
+    if (fixed) {
+      const int item = p >> (num_splits - 1);
+      sg.seq = unsigned(item) / unsigned(nkv), sg.kvh = item - sg.seq * nkv;
+      sg.tiles = tiles_of(sg.seq);
+      const int part = (sg.tiles + num_splits - 1) >> (num_splits - 1);
+      sg.first = num_splits == 2 && (p & 1) ? part : 0;
+      sg.n = min(part, sg.tiles - sg.first);
       return p + 1;
     }
     move_to(w, p);
@@ -178,7 +182,7 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
   // ---- this warp's tiles, one after the other over all segments: what is fetched next
   uint8_t* ring = smem + warp * (kDecStages * 2 * kTileBytes);
   Window fw{-32, 0, 0, 0};
-  if (p_begin < p_end && !whole) move_to(fw, p_begin);
+  if (p_begin < p_end && !fixed) move_to(fw, p_begin);
   Window cw = fw;
   Seg fs{};
   int fp = p_begin, fi = 0, f_tile0 = 0;
@@ -221,7 +225,7 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
     Seg sg;
     const int here = p;
     p = segment(p, cw, sg);
-    if (sg.n == 0) continue;                           // (a whole item: an empty sequence)
+    if (sg.n == 0 && num_splits == 1) continue;        // (an empty sequence; an empty half still has a record)
     const int len = seq_lens[sg.seq];
     const int first_tok = EXT && window > 0 ? max(0, len - window) : 0;
     uint32_t qb[NB][kSteps][2];
@@ -339,11 +343,11 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
         }
       }
     __syncthreads();
-    const int start = whole ? 0 : here - sg.first;               // position of the item's first tile
-    const int pieces = whole ? 1 : (start + sg.tiles - 1) / per - start / per + 1;
+    const int start = here - sg.first;                           // position of the item's first tile
+    const int pieces = fixed ? num_splits : (start + sg.tiles - 1) / per - start / per + 1;
     const bool alone = pieces == 1;
-    const int piece = alone ? 0 : int(blockIdx.x) - start / per;
-    if (!whole && sg.first == 0 && threadIdx.x < G)
+    const int piece = fixed ? int(blockIdx.x) & 1 : int(blockIdx.x) - start / per;
+    if (!fixed && sg.first == 0 && threadIdx.x < G)
       *piece_count(scratch, sg.seq * nh + sg.kvh * G + threadIdx.x, num_splits, HD) = pieces;
     constexpr int kPart = HD / 4;                                // a thread: four elements this far apart
 #pragma unroll 1
@@ -380,22 +384,22 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
   for (int i = blockIdx.x; i < num_seqs; i += gridDim.x)         // sequences of nothing: zeros
     if (tiles_of(i) == 0) {
       for (int d = threadIdx.x; d < nh * HD; d += blockDim.x) out[size_t(i) * ldo + d] = __float2half_rn(0.f);
-      if (!whole)
+      if (!fixed)
         for (int h = threadIdx.x; h < nh; h += blockDim.x) *piece_count(scratch, i * nh + h, num_splits, HD) = 1;
     }
 }
 
-// Items that attn_decode_kernel cut in pieces.  grid (nh, sequences), HD threads.
+// Items that attn_decode_kernel cut in pieces (num_splits > 1).  grid (nh, sequences), HD threads.
 template <int HD>
 __global__ void attn_combine_kernel(float* __restrict__ scratch, __half* __restrict__ out, int ldo, int nh, int num_splits) {
   pdl_launch_dependents();
   pdl_wait();
   const int head = blockIdx.x, seq = blockIdx.y, d = threadIdx.x;
   const float* src = scratch + size_t(seq * nh + head) * num_splits * (HD + 2);
-  // what a few pieces need is read beside their number, not behind it (num_splits >= 3: places that exist, whatever they hold);
-  // lane s has the maximum and the sum of piece s
-  const int lane = threadIdx.x & 31, some = num_splits - 1;
-  const int pieces = *piece_count(scratch, seq * nh + head, num_splits, HD);
+  // what a few pieces need is read beside their number, not behind it (places that exist, whatever they hold); lane s has the
+  // maximum and the sum of piece s
+  const int lane = threadIdx.x & 31, some = max(2, num_splits - 1);
+  const int pieces = num_splits == 2 ? 2 : *piece_count(scratch, seq * nh + head, num_splits, HD);
   float m = lane < some ? src[lane * (HD + 2) + HD] : -INFINITY, l = lane < some ? src[lane * (HD + 2) + HD + 1] : 0.f;
   float o[4];
 #pragma unroll
@@ -662,14 +666,14 @@ static int launch_decode(const void* q, int ldq, const void* kv, const void* bt,
   if ((1 << shift) != tpb) shift = -1;
   // cut: as many CTAs as the chip holds at once (rings of 48, 96 and 192 KB), each with the same share of the tiles
   const int fit = decode_sms() * (HD == 256 ? 1 : HD == 128 ? 2 : 4);
-  const int ctas = splits >= 3 ? min(fit, num_seqs * nkv * (splits - 1)) : num_seqs * nkv;   // (with few sequences most of the chip is left to the next kernel)
+  const int ctas = splits >= 3 ? min(fit, num_seqs * nkv * (splits - 1)) : num_seqs * nkv * splits;   // (with few sequences most of the chip is left to the next kernel)
   if (launch_pdl(attn_decode_kernel<HD, EXT, NB>, dim3(ctas), dim3(kDecWarps * 32), size_t(kDecodeSmem<HD, NB>), st,
                  reinterpret_cast<const __half*>(q), ldq, reinterpret_cast<const __half*>(kv), reinterpret_cast<const int*>(bt),
                  max_blocks, reinterpret_cast<const int*>(lens), reinterpret_cast<__half*>(out), ldo,
                  reinterpret_cast<float*>(scratch), num_seqs, nh, nkv, block_size, shift, splits, scale * kLog2e, blk_stride,
                  half_stride, softcap, window) != cudaSuccess)
     return ZSE_ERR_LAUNCH;
-  if (splits >= 3) {
+  if (splits > 1) {
     if (launch_pdl(attn_combine_kernel<HD>, dim3(nh, num_seqs), dim3(HD), 0, st, reinterpret_cast<float*>(scratch),
                    reinterpret_cast<__half*>(out), ldo, nh, splits) != cudaSuccess)
       return ZSE_ERR_LAUNCH;

@@ -7,6 +7,9 @@
 // such a caller for `zse_attn_decode_scratch_floats(...)` floats of scratch when num_splits > 1; this variant keeps
 // the scratch in a fixed array that is part of the library image on every device.
 //
+// num_splits.  1: a CTA per (sequence, kv head), no scratch.  2: two CTAs for each of them, half the tokens each.  N >= 3: all
+// CTAs take equal shares of all tokens, and a (sequence, kv head) is cut into at most N - 1 pieces.
+//
 // Limit.  The array holds ZSE_ATTN_STATIC_SCRATCH_FLOATS floats (16 MiB).  A call needs
 // num_seqs * nh * num_splits * (hd + 2) floats when num_splits > 1 and none when num_splits == 1; a call that needs
 // more returns ZSE_ERR_LIMIT and launches nothing.  zse_attn_decode_static_max_floats() returns the limit so that a
@@ -20,8 +23,8 @@
 // racing there write the same values, but nothing guarantees it).  A failed lookup returns ZSE_ERR_DRIVER and is
 // retried by the next call.  A call with num_splits == 1 needs no scratch and does no lookup.
 //
-// Sharing.  Every call on one device uses the same array.  Nothing in it has to start at zero: each call writes
-// every word it later reads.  Two calls that may run at the same time on one device (different streams without an
+// Sharing.  Every call on one device uses the same array.  Nothing in it has to start at zero: what a call reads of words
+// that it has not written does not reach a result.  Two calls that may run at the same time on one device (different streams without an
 // ordering between them) race on the array and produce wrong results; order them on one stream or with events.
 #pragma once
 #include <stdint.h>

@@ -145,7 +145,7 @@ extern "C" int zse_step_forward(const ZseStepModel* m, const ZseStepBuffers* b, 
     if (decode)
       p.did(zse_attn_decode(b->qkv, qkv_ld, kv_layer, b->block_tables, b->max_blocks, b->seq_lens, b->attn_out,
                             nh * hd, b->attn_scratch, num_seqs, nh, nkv, hd, block_size, attn_splits, m->scale, stream),
-            attn_splits >= 3 ? 2 : 1);
+            attn_splits > 1 ? 2 : 1);
     else if (m->attn_tc && hd == 128 && kv_blocks > 0)
       p.did(zse_attn_prefill_tc(b->qkv, qkv_ld, M, kv_layer, kv_blocks, b->block_tables, b->max_blocks, b->cu_q,
                                 b->q_pos0, b->attn_out, nh * hd, num_seqs, max_q_len, nh, nkv, hd, block_size, m->scale,

@@ -85,3 +85,24 @@ def test_decode_attention(hd, nh, nkv, bs, softcap, window, splits, lens):
 def test_many_pieces_and_many_sequences(splits, lens):
     """More pieces than a warp has lanes, more sequences than one window of 32, sequences of nothing in between."""
     test_decode_attention(128, 8, 2, 16, 0, 0, splits, lens)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lens", [[3000], [1, 0, 16, 17, 700]])
+def test_two_pieces_are_two(lens):
+    """num_splits = 2: half of every sequence in each record, whatever its length; the records add up to the output."""
+    from zse_b200.ops.backend import CudaOps
+    nh, nkv, hd, bs = 8, 2, 128, 16
+    ops, S = CudaOps("cuda"), len(lens)
+    q, kv, bt, ln = _case(S, nh, nkv, hd, bs, lens)
+    out = torch.full((S, nh * hd), 7.0, dtype=torch.float16, device="cuda")
+    scratch = torch.full((S, nh, 2, hd + 2), float("nan"), device="cuda")
+    ops.attn_decode(q, kv, bt, ln, out, S, nh, nkv, hd, bs, hd ** -0.5, scratch, 2)
+    torch.cuda.synchronize()
+    ops.check()
+    o, m, l = scratch[..., :hd].double(), scratch[..., hd].double(), scratch[..., hd + 1].double()
+    for s, n in enumerate(lens):
+        assert bool((l[s, :, 0] > 0).all()) == (n > 0) and bool((l[s, :, 1] > 0).all()) == (n > 16)
+    f = torch.where(l > 0, torch.exp2(m - m.amax(2, keepdim=True)), 0.0)
+    merged = (o * f[..., None]).sum(2) / (l * f).sum(2).clamp(min=1e-30)[..., None]
+    assert (out.view(S, nh, hd).double() - merged).abs().max() <= 2.0 ** -11 * merged.abs().max() + 1e-6

@@ -569,7 +569,7 @@ def attn_decode_ext(q, ldq, kv_layer, block_tables, seq_lens, out, ldo, scratch,
     _ck(load().zse_attn_decode_ext(_p(q), ldq, _p(kv_layer), kv_layer.stride(0), kv_layer.stride(1), _p(block_tables),
                                    block_tables.stride(0), _p(seq_lens), _p(out), ldo, _p(scratch), num_seqs, nh, nkv,
                                    hd, block_size, num_splits, float(scale), float(softcap), int(window), _stream()),
-        "attn_decode_ext")
+        "attn_decode_ext", 2 if num_splits > 1 else 1)
 
 
 def attn_prefill_ext(q, ldq, kv_layer, block_tables, cu_q, q_pos0, out, ldo, num_seqs, max_q_len, nh, nkv, hd,
