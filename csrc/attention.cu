@@ -63,8 +63,12 @@ __device__ __forceinline__ uint32_t tile_off(int row, int chunk) {
 // by attn_combine_kernel (at most num_splits - 1 pieces: `per` is raised for that if one sequence is very long).  The last of a
 // head's num_splits records in scratch says how many pieces there are.  That leaves nothing for two pieces, so with num_splits = 2
 // every item is cut in two halves; with 1 items stay whole.
+constexpr int kDecStages = 3;                                     // of a warp's ring
+// Where a warp's O goes when its item is merged: to a place of its own, or to the slot of its last tile, which lets one more CTA
+// onto an SM where there would be no room for it (HD = 64; NB = 2), but no warp may fetch on before all have read it (2 % where the
+// CTAs are the same).
 template <int HD, int NB>
-constexpr int kDecodeStages = HD == 256 && NB == 2 ? 2 : 3;       // of a warp's ring
+constexpr bool kOwnPlace = NB == 1 && HD >= 128;
 __device__ __forceinline__ int seq_tiles(int len, int window) {
   return ((len + 15) >> 4) - ((window > 0 ? max(0, len - window) : 0) >> 4);
 }
@@ -106,14 +110,21 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
                    float* __restrict__ scratch, int num_seqs, int nh, int nkv, int block_size, int block_shift,
                    int num_splits, float scale_log2, long long blk_stride, long long half_stride, float softcap, int window) {
   constexpr int kTileBytes = 16 * HD * 2;              // one 16-token K (or V) tile
-  constexpr int kDecStages = kDecodeStages<HD, NB>;
   constexpr int kChunksPerRow = HD / 8;
   constexpr int kSteps = HD / 16;
   constexpr int kHeads = 8 * NB;
-  constexpr int kPitch = HD + 4;                       // floats per head in the merge buffers: conflict-free
-  constexpr int kBuf = kHeads * kPitch + 2 * kHeads;   // O, then m and l per head
+  constexpr int kSlotBytes = 2 * kTileBytes;           // K and V
+  constexpr bool kOwn = kOwnPlace<HD, NB>;
+  constexpr int kPitch = kOwn ? HD + 4 : HD;           // floats per head of a warp's O
+  constexpr int kGiven = kHeads * kPitch;
+  static_assert(kOwn || kGiven * 4 <= kSlotBytes, "O fits a slot");
   extern __shared__ __align__(128) uint8_t smem[];
-  float* merge = reinterpret_cast<float*>(smem + kDecWarps * kDecStages * 2 * kTileBytes);      // a buffer per warp
+  struct Given {                                       // behind the rings, per warp: m, l, where O is
+    float m[kHeads], l[kHeads];
+    int slot;
+  };
+  Given* given = reinterpret_cast<Given*>(smem + kDecWarps * kDecStages * kSlotBytes);
+  float* own = reinterpret_cast<float*>(given + kDecWarps);
   pdl_launch_dependents();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t2 = (lane & 3) * 2;
@@ -180,7 +191,7 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
   };
 
   // ---- this warp's tiles, one after the other over all segments: what is fetched next
-  uint8_t* ring = smem + warp * (kDecStages * 2 * kTileBytes);
+  uint8_t* ring = smem + warp * (kDecStages * kSlotBytes);
   Window fw{-32, 0, 0, 0};
   if (p_begin < p_end && !fixed) move_to(fw, p_begin);
   Window cw = fw;
@@ -202,7 +213,7 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
       if (blk >= 0) {
         const __half* ksrc = kv + size_t(blk) * blk_stride + (size_t(fs.kvh) * block_size + in * 16) * HD + lane * 8;
         const __half* vsrc = ksrc + half_stride;
-        uint8_t* kd = ring + slot * 2 * kTileBytes;
+        uint8_t* kd = ring + slot * kSlotBytes;
 #pragma unroll
         for (int j = 0; j < kTileBytes / 512; ++j) {
           const int idx = j * 32 + lane;
@@ -252,7 +263,7 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
       __syncwarp();
       const bool hole = (holes >> slot) & 1u;
       issue(slot == 0 ? kDecStages - 1 : slot - 1);    // the slot of the tile before this one
-      const uint32_t kbase = smem_u32(ring + slot * 2 * kTileBytes), vbase = kbase + kTileBytes;
+      const uint32_t kbase = smem_u32(ring + slot * kSlotBytes), vbase = kbase + kTileBytes;
       slot = slot + 1 == kDecStages ? 0 : slot + 1;
       if (hole) continue;
       const int tok = ((first_tok >> 4) + sg.first + i) << 4;
@@ -325,23 +336,26 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
       for (int e = 0; e < 2; ++e)
 #pragma unroll
         for (int sh = 4; sh < 32; sh <<= 1) l[nb][e] += __shfl_xor_sync(0xffffffffu, l[nb][e], sh);
-    __syncthreads();                                   // (the item before has been read)
-    float* mine = merge + warp * kBuf;
+    // (conflict-free: heads four banks apart, or bits 3 and 4 of a column turned by the head)
+    const int mine = slot == 0 ? kDecStages - 1 : slot - 1;      // the slot of the last tile
+    if (kOwn) __syncthreads(); else __syncwarp();                // (own places: the item before has been read)
+    float* to = kOwn ? own + warp * kGiven : reinterpret_cast<float*>(ring + mine * kSlotBytes);
 #pragma unroll
     for (int nb = 0; nb < NB; ++nb)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int h = nb * 8 + t2 + e;
+        const int h = nb * 8 + t2 + e, turn = kOwn ? 0 : (h & 6) << 2;
 #pragma unroll
         for (int d = 0; d < kSteps; ++d) {
-          mine[h * kPitch + d * 16 + g] = o[nb][d][e];
-          mine[h * kPitch + d * 16 + g + 8] = o[nb][d][2 + e];
+          to[h * kPitch + ((d * 16 + g) ^ turn)] = o[nb][d][e];
+          to[h * kPitch + ((d * 16 + g + 8) ^ turn)] = o[nb][d][2 + e];
         }
         if (g == 0) {
-          mine[kHeads * kPitch + h] = m[nb][e];
-          mine[kHeads * kPitch + kHeads + h] = l[nb][e];
+          given[warp].m[h] = m[nb][e];
+          given[warp].l[h] = l[nb][e];
         }
       }
+    if (!kOwn && lane == 0) given[warp].slot = mine;
     __syncthreads();
     const int start = here - sg.first;                           // position of the item's first tile
     const int pieces = fixed ? num_splits : (start + sg.tiles - 1) / per - start / per + 1;
@@ -355,14 +369,16 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
       const int h = idx / kPart, d = idx % kPart, head = sg.kvh * G + h;
       float mw[kDecWarps], M = -INFINITY, L = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int w = 0; w < kDecWarps; ++w) M = fmaxf(M, mw[w] = merge[w * kBuf + kHeads * kPitch + h]);
+      for (int w = 0; w < kDecWarps; ++w) M = fmaxf(M, mw[w] = given[w].m[h]);
 #pragma unroll
       for (int w = 0; w < kDecWarps; ++w) {
-        const float* src = merge + w * kBuf;
+        const float* src =
+            (kOwn ? own + w * kGiven : reinterpret_cast<const float*>(smem + (w * kDecStages + given[w].slot) * kSlotBytes)) +
+            h * kPitch;
         const float f = mw[w] == -INFINITY ? 0.f : ex2_approx(mw[w] - M);
-        L += src[kHeads * kPitch + kHeads + h] * f;
+        L += given[w].l[h] * f;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) acc[k] += src[h * kPitch + d + k * kPart] * f;
+        for (int k = 0; k < 4; ++k) acc[k] += src[(d + k * kPart) ^ (kOwn ? 0 : (h & 6) << 2)] * f;
       }
       if (alone) {
         __half* dst = out + size_t(sg.seq) * ldo + size_t(head) * HD + d;
@@ -379,6 +395,7 @@ attn_decode_kernel(const __half* __restrict__ q, int ldq, const __half* __restri
         }
       }
     }
+    if (!kOwn) __syncthreads();
   }
   cp_async_wait<0>();
   for (int i = blockIdx.x; i < num_seqs; i += gridDim.x)         // sequences of nothing: zeros
@@ -625,9 +642,15 @@ extern "C" int64_t zse_attn_decode_scratch_floats(int num_seqs, int nh, int hd, 
   return int64_t(num_seqs) * nh * max_splits * (hd + 2);
 }
 
-// Shared memory of the decode kernel: rings and a merge buffer per warp.
+// Shared memory of the decode kernel: rings, and what its warps give besides O.
 template <int HD, int NB>
-constexpr int kDecodeSmem = kDecWarps * (kDecodeStages<HD, NB> * 2 * 16 * HD * 2 + (8 * NB * (HD + 4) + 2 * 8 * NB) * 4);
+constexpr int kDecodeSmem =
+    kDecWarps * (kDecStages * 2 * 16 * HD * 2 + (2 * 8 * NB + 1) * 4 + (kOwnPlace<HD, NB> ? 8 * NB * (HD + 4) * 4 : 0));
+// CTAs that an SM holds: shared memory decides (228 KB, 1 KB of each CTA's is the system's; 255 registers a thread leave room for two)
+template <int HD, int NB>
+constexpr int kDecodeCtasPerSm = 228 * 1024 / (kDecodeSmem<HD, NB> + 1024);
+static_assert(kDecodeCtasPerSm<64, 1> == 4 && kDecodeCtasPerSm<64, 2> == 4 && kDecodeCtasPerSm<128, 1> == 2 &&
+              kDecodeCtasPerSm<128, 2> == 2 && kDecodeCtasPerSm<256, 1> == 1 && kDecodeCtasPerSm<256, 2> == 1);
 
 // The attribute is raised once per device (host work: not a stream operation).
 template <int HD, bool EXT, int NB>
@@ -664,9 +687,10 @@ static int launch_decode(const void* q, int ldq, const void* kv, const void* bt,
   int shift = 0;
   while ((1 << shift) < tpb) ++shift;
   if ((1 << shift) != tpb) shift = -1;
-  // cut: as many CTAs as the chip holds at once (rings of 48, 96 and 192 KB), each with the same share of the tiles
-  const int fit = decode_sms() * (HD == 256 ? 1 : HD == 128 ? 2 : 4);
-  const int ctas = splits >= 3 ? min(fit, num_seqs * nkv * (splits - 1)) : num_seqs * nkv * splits;   // (with few sequences most of the chip is left to the next kernel)
+  // cut: as many CTAs as the chip holds at once, each with the same share of the tiles (with few sequences most of the chip is left
+  // to the next kernel)
+  const int fit = decode_sms() * kDecodeCtasPerSm<HD, NB>;
+  const int ctas = splits >= 3 ? min(fit, num_seqs * nkv * (splits - 1)) : num_seqs * nkv * splits;
   if (launch_pdl(attn_decode_kernel<HD, EXT, NB>, dim3(ctas), dim3(kDecWarps * 32), size_t(kDecodeSmem<HD, NB>), st,
                  reinterpret_cast<const __half*>(q), ldq, reinterpret_cast<const __half*>(kv), reinterpret_cast<const int*>(bt),
                  max_blocks, reinterpret_cast<const int*>(lens), reinterpret_cast<__half*>(out), ldo,
