@@ -302,16 +302,22 @@ class DecoderModel:
     def stage_prefill(self, b: StepBuffers, spans) -> None:
         """Called while a packed pass is staged; ``spans[s] = (start, tokens)`` in the pass's order."""
 
-    def attention_splits(self, seqs: int, max_len: int, most: int, sms: int) -> int:
-        """Bound on the pieces that a sequence may be cut into in a decode step over ``seqs`` sequences of up to ``max_len``
-        tokens (few distinct values: each is a CUDA graph of its own).  The kernel gives every CTA an equal share of all tokens
-        and merges what it had to cut; pieces have 64 tokens at least.  With four (sequence, kv head) items an SM the hardware's
-        own order of whole items is as good and there is nothing to merge (7B, 160 sequences of 64 to 1100 tokens: 48 us whole,
-        45 us and a merge of 5 cut)."""
-        if seqs * self.plan.num_kv_heads >= 4 * sms:
+    def attention_splits(self, seqs: int, max_len: int, most: int, sms: int, tokens: Optional[int] = None) -> int:
+        """``num_splits`` of the decode kernel for a step over ``seqs`` sequences of up to ``max_len`` tokens, ``tokens`` in all (not
+        given: all as long): 1 keeps every (sequence, kv head) in one CTA, ``most`` cuts all tokens into equal shares.  The kernel
+        cuts by the lengths that it finds on the device, so there is no third value, and no third CUDA graph of a batch size.
+
+        Cutting costs about 3.5 us a layer for the merge.  Without it the step waits for its longest sequence, which one CTA reads
+        at 100 tokens of 128 a us, while all CTAs read some 7700; the longest has company for a good part of that time.  Measured
+        (whole | cut, us a step): 7B, 1 x 300 tokens 1697 | 1714, 1 x 1000 1902 | 1734, 17 x 100 2410 | 2506, 32 x 300 2497 | 2604, 17 of
+        100 to 3000 3311 | 2727, 100 of 64 to 900 3489 | 3701; 14B, of 128 to 2300 tokens: 16 5201 | 4748, 32 5642 | 5696, 64 7539 |
+        7763."""
+        if most < 2:
             return 1
-        n = int(max(1, min(max_len // 64, most)))
-        return 1 << (n.bit_length() - 1)              # powers of two
+        width = self.config.head_dim / 128
+        whole = max_len * width / 100
+        alone = (seqs * max_len if tokens is None else tokens) * self.plan.num_kv_heads * width / 7700
+        return most if whole > 3.5 + 0.6 * alone * 148 / sms else 1
 
     # ---- forward --------------------------------------------------------------------------------------
     def _add_norm(self, b: StepBuffers, planes: int, weight: torch.Tensor, M: int, add=None) -> None:

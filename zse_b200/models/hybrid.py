@@ -282,7 +282,7 @@ class HybridModel(DesignModel):
             v = self._views[key] = PagedHeads(kv[run.cache_layer], attention_of(run.layer.spec), self.means_at)
         return v
 
-    def attention_splits(self, seqs: int, max_len: int, most: int, sms: int) -> int:
+    def attention_splits(self, seqs: int, max_len: int, most: int, sms: int, tokens: Optional[int] = None) -> int:
         if not self.heads_specs:
             return 1
         span = max(min(max_len, s.chunk or max_len, s.window + s.keep_first if s.window else max_len)

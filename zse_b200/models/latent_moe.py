@@ -191,7 +191,7 @@ class LatentMoEModel(DesignModel):
             self._row_views[key] = v
         return v
 
-    def attention_splits(self, seqs: int, max_len: int, most: int, sms: int) -> int:
+    def attention_splits(self, seqs: int, max_len: int, most: int, sms: int, tokens: Optional[int] = None) -> int:
         span = min(max_len, self.max_window) if self.max_window else max_len
         return attention_splits(seqs, max((L.spec.heads + 31) // 32 for L in self.layers), span, most, sms)
 

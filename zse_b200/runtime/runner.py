@@ -278,10 +278,10 @@ class ModelRunner:
         return (toks, b.logits[:n_rows]) if all_logits else toks
 
     # ---- batched decode -----------------------------------------------------------------------------------
-    def _pick_splits(self, S: int, max_len: int) -> int:
+    def _pick_splits(self, S: int, max_len: int, tokens: int) -> int:
         if self.device.type != "cuda":
             return 1
-        return self.model.attention_splits(S, max_len, self.max_attn_splits, self._sm)
+        return self.model.attention_splits(S, max_len, self.max_attn_splits, self._sm, tokens)
 
     def _apply_penalties(self, penalties, n_rows: int) -> None:
         """``penalties[i] = (penalty, {token: count})`` for logits row i (zse-engine/zse_engine/orchestrator/
@@ -349,7 +349,7 @@ class ModelRunner:
             self._stage_states([(sid, int(p), 1) for sid, p in zip(seq_ids, n_["pos"][:S])], Sp)
         greedy = self._stage_sampling(sampling or [GREEDY] * S, Sp)
         self._staging_end()
-        splits = self._pick_splits(Sp, max_len)
+        splits = self._pick_splits(Sp, max_len, int(n_["lens"][:S].sum()))
         self._step += 1
         counter = self._launch_counter()
         before = counter[0]
