@@ -36,3 +36,14 @@ def test_bounds_of_the_cut():
 
 def test_models_without_paged_heads_take_the_number_of_tokens_too():
     assert HybridModel.attention_splits(types.SimpleNamespace(heads_specs=[]), 1, 100, 16, 148, 100) == 1
+
+
+@pytest.mark.parametrize("sharded,rows", [(False, {1: 1, 5: 8, 65: 96, 96: 96, 97: 128, 130: 160, 161: 192, 193: 256, 256: 256}),
+                                          (True, {1: 1, 5: 8, 65: 128, 96: 128, 97: 128, 130: 256, 161: 256, 256: 256})])
+def test_rows_of_the_graph(sharded, rows):
+    """A sharded model's step keeps the rows, and so the exchange, of the next power of two."""
+    runner = types.SimpleNamespace(model=types.SimpleNamespace(comm=object() if sharded else None), max_batch_seqs=256,
+                                   DECODE_BUCKETS=ModelRunner.DECODE_BUCKETS, SHARDED_BUCKETS=ModelRunner.SHARDED_BUCKETS)
+    assert {n: ModelRunner._graph_rows(runner, n) for n in rows} == rows
+    runner.max_batch_seqs = 80
+    assert ModelRunner._graph_rows(runner, 70) == 80

@@ -47,6 +47,9 @@ def _bucket(n: int, buckets: Sequence[int]) -> int:
 
 class ModelRunner:
     DECODE_BUCKETS = (1, 2, 4, 8, 16, 32, 64, 96, 128, 160, 192, 256)
+    # Sharded models: what exchanges the rows of a pass between the ranks is chosen by their number (ZSE_TP_FUSED_SP_ROWS,
+    # ZSE_TP_NCCL_ROWS), by measurements at powers of two, and 96 rows would not take the exchange of 128.
+    SHARDED_BUCKETS = (1, 2, 4, 8, 16, 32, 64, 128, 256)
 
     def __init__(self, model: DecoderModel, cache: KVCacheManager, max_batch_seqs: int = 64,
                  max_tokens_per_pass: int = 2048, max_seq_len: Optional[int] = None, use_graphs: Optional[bool] = None,
@@ -278,6 +281,11 @@ class ModelRunner:
         return (toks, b.logits[:n_rows]) if all_logits else toks
 
     # ---- batched decode -----------------------------------------------------------------------------------
+    def _graph_rows(self, S: int) -> int:
+        """Rows of the CUDA graph that a step of ``S`` sequences runs in."""
+        buckets = self.DECODE_BUCKETS if self.model.comm is None else self.SHARDED_BUCKETS
+        return min(_bucket(S, buckets), self.max_batch_seqs)
+
     def _pick_splits(self, S: int, max_len: int, tokens: int) -> int:
         if self.device.type != "cuda":
             return 1
@@ -316,7 +324,7 @@ class ModelRunner:
             return (lambda: []) if defer else []
         if S > self.max_batch_seqs:
             raise ValueError(f"decode batch {S} exceeds max_batch_seqs {self.max_batch_seqs}")
-        Sp = min(_bucket(S, self.DECODE_BUCKETS), self.max_batch_seqs) if self.use_graphs else S
+        Sp = self._graph_rows(S) if self.use_graphs else S
         bs = cache.block_size
         n_ = self._np
         self._staging_begin()
@@ -544,7 +552,7 @@ class ModelRunner:
         if not self.use_graphs:
             return 0
         base = 1_000_100_000
-        for m in sorted({min(_bucket(int(x), self.DECODE_BUCKETS), self.max_batch_seqs) for x in batch_sizes}):
+        for m in sorted({self._graph_rows(int(x)) for x in batch_sizes}):
             sids = list(range(base, base + m))
             made = []
             try:
