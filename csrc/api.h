@@ -29,8 +29,9 @@ int zse_gemm_w4_splits(int M, int N, int K, int k_split);
 int zse_gemm_w8(const void* w_tiled, const void* x, int x_rows_cap, const void* bias, void* out, int M, int N, int K,
                 int ldo, int epilogue, int k_split, void* status, void* stream);
 int zse_gemm_w8_splits(int M, int N, int K, int k_split);
-// the launcher's plan for a call: out4 = {tiles per wide CTA, K splits, cluster size, CTA shape: 0 wide, 1 narrow,
-// -1 gemm_w4_small.cu}
+// k_split: planes of epilogue 2; a cluster of so many CTAs along K on the others (0: the launcher decides).
+// The launcher's plan for a call: out4 = {tiles per wide CTA, K splits, cluster size along K, kind: 0 wide CTAs, 1 narrow CTAs, -1
+// gemm_w4_small.cu, 2 gemm_pair.cu (its first number: tokens of a unit)}
 void zse_gemm_w4_plan(int M, int N, int K, int epilogue, int k_split, int sm_count, int* out4);
 // ---- gemm_w4_dec.cu -----------------------------------------------------------------------------------------
 // Decode-sized INT4 GEMM (M <= 64): one persistent CTA per SM over an even split of the weight stream.

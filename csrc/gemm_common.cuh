@@ -114,6 +114,7 @@ int gemm_w4_small_run(const void* w_tiled, const void* x, const void* bias, void
 int gemm_pair_run(bool w8, const void* w_tiled, const void* x, int x_rows_cap, const void* bias, void* out, int M, int N,
                   int K, int ldo, int epilogue, int want_split, const GatherWait* gather, Status* status, cudaStream_t st);
 int gemm_pair_planes(int M, int N, int K, int want_split);
+void gemm_pair_plan(int M, int N, int K, int epilogue, int want_split, int sm_count, int* tokens, int* splits);
 
 inline int pick_nt(int M) {
   if (M <= 16) return 16;

@@ -584,6 +584,12 @@ int gemm_pair_planes(int M, int N, int K, int want_split) {
   return plan_pair(M, N, K, true, pair_n_tiles(N, kEpiPartialF32), pair_sm_count(), want_split).ks;
 }
 
+void gemm_pair_plan(int M, int N, int K, int epilogue, int want_split, int sm_count, int* tokens, int* splits) {
+  const PairPlan p = plan_pair(M, N, K, epilogue == kEpiPartialF32, pair_n_tiles(N, epilogue), sm_count, want_split);
+  *tokens = p.nt;
+  *splits = p.ks;
+}
+
 int gemm_pair_run(bool w8, const void* w_tiled, const void* x, int x_rows_cap, const void* bias, void* out, int M, int N,
                   int K, int ldo, int epilogue, int want_split, const GatherWait* gather, Status* status, cudaStream_t st) {
   if (M <= 0) return 0;

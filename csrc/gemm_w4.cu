@@ -936,9 +936,10 @@ static bool takes_small(int M, int N, int K, int epilogue, int k_split) {
 // More than 64 tokens: gemm_pair.cu, except for narrow layers whose epilogue needs the whole sum.  They leave most pairs without
 // work, and a cluster along K of this file's wide CTA adds the parts on chip.  The line lies between 14 pairs of tiles (Gemma-2 9B
 // o_proj, 128 tokens: 17.4 us here, 23.4 there; down_proj 35.7, 53.2) and 18 (7B QKV, 128 tokens: 27.6 us here, 22.5 there), and at
-// 256 tokens (o_proj, 320 tokens: 27.6, 24.6).
-static bool takes_pair(int M, int N, int epilogue, int sm_count) {
-  if (M <= 64) return false;
+// 256 tokens (o_proj, 320 tokens: 27.6, 24.6).  Layers of 15 to 17 pairs were not measured.  An explicit split of a whole-sum epilogue is a
+// cluster along K, which only this file has.
+static bool takes_pair(int M, int N, int epilogue, int k_split, int sm_count) {
+  if (M <= 64 || (epilogue != kEpiPartialF32 && k_split > 1)) return false;
   const int pairs = ((epilogue == kEpiSwiGLU ? (N / 2 + 63) / 64 : (N + kTileN - 1) / kTileN) + 1) / 2;
   return epilogue == kEpiPartialF32 || M > 256 || 5 * pairs > sm_count / 2;
 }
@@ -959,7 +960,7 @@ static int run_gemm_w4(const void* w_tiled, const void* x, int x_rows_cap, const
   if (push == nullptr && takes_small(M, N, K, epilogue, k_split))
     return gemm_w4_small_run(w_tiled, x, bias, out, M, N, K, ldo, epilogue, k_split, nullptr,
                              reinterpret_cast<cudaStream_t>(stream));
-  if (push == nullptr && sp == nullptr && takes_pair(M, N, epilogue, sm_count))
+  if (push == nullptr && sp == nullptr && takes_pair(M, N, epilogue, k_split, sm_count))
     return gemm_pair_run(false, w_tiled, x, x_rows_cap, bias, out, M, N, K, ldo, epilogue, k_split, gather,
                          reinterpret_cast<Status*>(status), reinterpret_cast<cudaStream_t>(stream));
   const int k_stages = K / kW4StageK;
@@ -1082,12 +1083,17 @@ extern "C" int zse_gemm_w4_max_clusters(int narrow, int cluster) {
   return n;
 }
 
-// What the launcher would do for these arguments: out4 = {weight tiles per wide CTA, K splits, cluster size along K,
-// CTA shape (0 wide, 1 narrow)}; -1 in out4[3] = gemm_w4_small.cu.
+// What the launcher does with these arguments: out4 = {weight tiles per wide CTA, K splits, cluster size along K, kind}, kind 0 wide
+// CTAs, 1 narrow CTAs, -1 gemm_w4_small.cu, 2 gemm_pair.cu (out4[0]: tokens of a unit).
 extern "C" void zse_gemm_w4_plan(int M, int N, int K, int epilogue, int k_split, int sm_count, int* out4) {
   if (sm_count <= 0) sm_count = 148;
   if (takes_small(M, N, K, epilogue, k_split)) {
     out4[0] = 1, out4[1] = epilogue == kEpiPartialF32 ? gemm_w4_small_planes(N, K, k_split) : 1, out4[2] = 1, out4[3] = -1;
+    return;
+  }
+  if (takes_pair(M, N, epilogue, k_split, sm_count)) {
+    gemm_pair_plan(M, N, K, epilogue, k_split, sm_count, &out4[0], &out4[1]);
+    out4[2] = 1, out4[3] = 2;
     return;
   }
   plan_w4(M, N, K, epilogue, sm_count, k_split, &out4[0], &out4[1], &out4[2], &out4[3]);

@@ -85,3 +85,23 @@ def test_pair_planes_on_request(ops, ks):
     ops.check()
     assert n == native.gemm_w4_splits(M, N, K, ks) and n <= ks
     assert _rel(planes[:n].double().sum(0), x.float() @ wd.float().T) < 1e-5
+
+
+@pytest.mark.parametrize("ks", [2, 4])
+@pytest.mark.parametrize("M,N,K,epilogue", [(200, 1024, 2048, 0), (300, 2048, 1152, 0), (513, 2048, 640, 1)])
+def test_cluster_along_k_on_request(ops, ks, M, N, K, epilogue):
+    """An explicit split of an epilogue that needs the whole sum: wide CTAs in a cluster along K (csrc/gemm_w4.cu)."""
+    assert native.gemm_w4_plan(M, N, K, epilogue, ks)[2:] == (ks, 0)
+    if epilogue == 1:
+        (g, gd), (u, ud) = _part("int4", N // 2, K, 1), _part("int4", N // 2, K, 2)
+        w, cols = ops.make_linear([g, u], K, 128, swiglu=True), N // 2
+    else:
+        p, wd = _part("int4", N, K, 3)
+        w, cols = ops.make_linear([p], K, 128), N
+    x = (torch.randn(M, K, device="cuda") * 0.5).half()
+    out = torch.full((M + 1, cols), 7.0, dtype=torch.float16, device="cuda")
+    native.gemm_w4(w.data, x, M, None, out, M, N, K, cols, epilogue, ks, ops.status.ptr)
+    torch.cuda.synchronize()
+    ops.check()
+    want = ref.swiglu(x.float() @ gd.float().T, x.float() @ ud.float().T) if epilogue == 1 else x.float() @ wd.float().T
+    assert _rel(out[:M], want) < 5e-4 and (out[M:] == 7).all()

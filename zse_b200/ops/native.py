@@ -443,7 +443,7 @@ def gemm_w4_dec_small(M, N, K, epilogue) -> bool:
 
 def gemm_w4_plan(M, N, K, epilogue, k_split=0, sm_count=148):
     """What ``gemm_w4`` does for a call: (tiles per wide CTA, K splits, cluster size, kind: 0 wide CTAs, 1 narrow CTAs, -1
-    csrc/gemm_w4_small.cu)."""
+    csrc/gemm_w4_small.cu, 2 csrc/gemm_pair.cu, whose first number is the tokens of a unit)."""
     out = (c_int * 4)()
     load().zse_gemm_w4_plan(M, N, K, epilogue, k_split, sm_count, out)
     return tuple(out)
