@@ -843,8 +843,9 @@ static int launch_w4_epi(int epilogue, const CUtensorMap& tx, const W4Args& a, d
   return ZSE_ERR_SHAPE;
 }
 
-// 0 = the planner decides, 1 = wide CTAs only, 2 = narrow (two per SM) CTAs wherever they are allowed;
-// adding 4 keeps calls of up to 8 tokens on the kernels of this file instead of gemm_w4_small.cu
+// 0 = the planner decides, 1 = wide CTAs only, 2 = narrow (two per SM) CTAs wherever they are allowed (planes of more than 64 tokens
+// are gemm_pair.cu's in any mode); anything but 0 keeps calls of up to 8 tokens out of gemm_w4_small.cu, 4 does only that, 8 gives
+// gemm_pair.cu every call of more than 64 tokens that it can take
 int g_w4_mode = 0;
 
 // How the launcher tiles a problem: weight tiles per CTA (R) and K splits (ks).  Measured on B200: a tcgen05.mma of
@@ -922,7 +923,7 @@ using namespace zse;
 static long long* g_w4_timing = nullptr;
 // Debug hook (only meaningful in builds with ZSE_W4_TIMING): device buffer of 20 x 8 counters.
 extern "C" void zse_gemm_w4_set_timing(void* dev_buffer) { g_w4_timing = reinterpret_cast<long long*>(dev_buffer); }
-// Tuning hook: 0 = planner decides between wide and narrow CTAs, 1 = wide only, 2 = narrow wherever allowed.
+// Tuning hook, see g_w4_mode.
 extern "C" void zse_gemm_w4_set_mode(int mode) { zse::g_w4_mode = mode; }
 
 // Up to 8 tokens: gemm_w4_small.cu, unless a tuning mode or a cluster along K asks for a CTA of this file or the layer is narrow
@@ -940,6 +941,7 @@ static bool takes_small(int M, int N, int K, int epilogue, int k_split) {
 // cluster along K, which only this file has.
 static bool takes_pair(int M, int N, int epilogue, int k_split, int sm_count) {
   if (M <= 64 || (epilogue != kEpiPartialF32 && k_split > 1)) return false;
+  if (epilogue != kEpiPartialF32 && g_w4_mode != 0 && g_w4_mode != 4) return (g_w4_mode & 8) != 0;
   const int pairs = ((epilogue == kEpiSwiGLU ? (N / 2 + 63) / 64 : (N + kTileN - 1) / kTileN) + 1) / 2;
   return epilogue == kEpiPartialF32 || M > 256 || 5 * pairs > sm_count / 2;
 }

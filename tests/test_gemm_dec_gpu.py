@@ -225,3 +225,28 @@ def test_int8_gate_up_with_swiglu(ops, ws, M, I, K):
     ops.check()
     want = ref.swiglu(x.float() @ gd.T, x.float() @ ud.T)
     assert _rel(out, want) < 3e-3, _rel(out, want)
+
+
+# Up to 8 tokens of INT4 are csrc/gemm_w4_small.cu's unless a layer is narrow and deep: these run the same cases in the persistent
+# kernel itself, which takes what the small one leaves and every projection with an exchange behind it.
+@pytest.fixture
+def no_small_kernel():
+    native.gemm_w4_set_mode(4)
+    yield
+    native.gemm_w4_set_mode(0)
+
+
+@pytest.mark.parametrize("M,N,K", [s for s in SHAPES if s[0] <= 8] + [(8, 1024, 8192), (2, 1280, 8192)])
+def test_few_tokens_in_this_kernel(ops, ws, no_small_kernel, M, N, K):
+    assert not native.gemm_w4_dec_small(M, N, K, 0) and not native.gemm_w4_dec_small(M, N, K, 2)
+    test_dec_fp16_and_fp32_epilogues(ops, ws, M, N, K)
+
+
+@pytest.mark.parametrize("M,I,K", [(1, 128, 256), (5, 256, 128), (8, 9664, 384)])
+def test_few_tokens_swiglu_in_this_kernel(ops, ws, no_small_kernel, M, I, K):
+    test_dec_swiglu(ops, ws, M, I, K)
+
+
+@pytest.mark.parametrize("M,nh,nkv,K,bs", [(1, 4, 1, 512, 16), (7, 5, 1, 640, 16), (4, 1, 1, 128, 16)])
+def test_few_tokens_qkv_in_this_kernel(ops, ws, no_small_kernel, M, nh, nkv, K, bs):
+    test_dec_qkv_rope_kv_write(ops, ws, M, nh, nkv, K, bs)

@@ -105,3 +105,24 @@ def test_cluster_along_k_on_request(ops, ks, M, N, K, epilogue):
     ops.check()
     want = ref.swiglu(x.float() @ gd.float().T, x.float() @ ud.float().T) if epilogue == 1 else x.float() @ wd.float().T
     assert _rel(out[:M], want) < 5e-4 and (out[M:] == 7).all()
+
+
+# Narrow layers of up to 256 tokens run in the wide CTA of csrc/gemm_w4.cu; these send them to the paired kernel, where the edges
+# of its tiles are.
+@pytest.fixture
+def pairs_only():
+    native.gemm_w4_set_mode(8)
+    yield
+    native.gemm_w4_set_mode(0)
+
+
+@pytest.mark.parametrize("M,N,K", [(65, 256, 128), (77, 384, 640), (160, 1000, 1152), (129, 100, 256), (256, 1920, 384)])
+def test_pair_narrow_int4(ops, pairs_only, M, N, K):
+    assert native.gemm_w4_plan(M, N, K, 0)[3] == native.gemm_w4_plan(M, N, K, 2)[3] == 2
+    test_pair_epilogues(ops, "int4", M, N, K)
+
+
+@pytest.mark.parametrize("M,I,K", [(66, 64, 256), (130, 200, 640), (255, 832, 128)])
+def test_pair_narrow_swiglu_int4(ops, pairs_only, M, I, K):
+    assert native.gemm_w4_plan(M, 2 * I, K, 1)[3] == 2
+    test_pair_swiglu(ops, "int4", M, I, K)

@@ -135,3 +135,19 @@ def test_small_infinite_activation(ops, M, N, K):
         ok = col != 0
         assert int(ok.sum()) > N // 2 and torch.equal(out[m][ok].float(), 65504 * sign[ok])
         assert torch.equal(planes[:n, m].sum(0)[ok], float("inf") * sign[ok])
+
+
+@pytest.mark.parametrize("M", [1, 8])
+@pytest.mark.parametrize("N,K", [(1024, 8192), (200, 6400), (3584, 14336)])
+def test_narrow_and_deep_layers(ops, M, N, K):
+    """Layers that the register-streamed kernel leaves to a cluster along K; the planes of the same layers are its own."""
+    assert native.gemm_w4_plan(M, N, K, 0)[3] != -1 and native.gemm_w4_plan(M, N, K, 2)[3] == -1
+    p, wd = _part(N, K, 5)
+    bias = (torch.randn(N, device="cuda") * 0.1).half()
+    x = (torch.randn(M, K, device="cuda") * 0.5).half()
+    out = torch.full((M + 1, N), 7.0, dtype=torch.float16, device="cuda")
+    ops.linear(ops.make_linear([p], K, 128, bias), x, M, out)
+    torch.cuda.synchronize()
+    ops.check()
+    # weights and the result rounded to fp16: 2^-11 each at most
+    assert _rel(out[:M], x.double() @ wd.T + bias.double()) < 1e-3 and (out[M:] == 7).all()

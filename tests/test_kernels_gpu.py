@@ -182,8 +182,8 @@ def test_gemm_w4_wide_and_narrow_ctas_agree(ops, mode, M, N, K, epi):
 @pytest.mark.parametrize("M,N,K,epi", [(1, 9472, 3584, "swiglu"), (2, 9472, 1024, "swiglu"), (2, 12288, 1024, "f16"),
                                        (1, 3584, 18944, "partial"), (2, 5120, 5120, "partial"),
                                        (1, 152064 // 8, 512, "f16")])
-def test_gemv_w4_one_and_two_tokens(ops, M, N, K, epi):
-    """CUDA-core GEMV path (taken for one or two tokens) against the oracle and against the tensor-core kernel."""
+def test_gemm_w4_one_and_two_tokens(ops, M, N, K, epi):
+    """One or two tokens (csrc/gemm_w4_small.cu) against the oracle and against the tcgen05 kernels."""
     from zse_b200.ops import native
     x = (torch.randn(M, K, device="cuda") * 0.5).half()
 
@@ -214,7 +214,7 @@ def test_gemv_w4_one_and_two_tokens(ops, M, N, K, epi):
     torch.cuda.synchronize()
     ops.check()
     assert _rel(got, want) < 3e-3, _rel(got, want)
-    native.gemm_w4_set_mode(4)                  # same call on the tensor cores
+    native.gemm_w4_set_mode(4)                  # the same call on the tcgen05 kernels, by the plain and by the decode entry
     try:
         tc = run()
         torch.cuda.synchronize()

@@ -1038,8 +1038,9 @@ def device_info() -> dict:
 
 
 def gemm_w4_set_mode(mode: int) -> None:
-    """Tuning hook for the INT4 GEMM: 0 = the planner picks the CTA shape, 1 = wide CTAs only, 2 = narrow CTAs (two per
-    SM) wherever they are allowed."""
+    """Tuning hook for the INT4 GEMM: 0 = the planner picks the kernel, 1 = wide CTAs only, 2 = narrow CTAs (two per SM)
+    wherever they are allowed, 4 = csrc/gemm_w4_small.cu is not used (nor is it with any other value but 0), 8 = csrc/gemm_pair.cu
+    for every call of more than 64 tokens."""
     load().zse_gemm_w4_set_mode(int(mode))
 
 
