@@ -25,7 +25,7 @@
 // (both), acc_empty (leader: 16 warps of each CTA have read their part).  The weight ring's depth is a multiple of four, so
 // that a slot is always read by the same group.
 //
-// Measured (B200, cold L2, one-CTA kernel before -> this one): 14B gate/up 2048 tokens 524 -> 385 us (1506 TFLOP/s, 0.93 of the
+// Measured (B200, cold L2, one-CTA kernel before -> this one): 14B gate/up 2048 tokens 524 -> 385 us (1506 TFLOP/s, 0.90 of the
 // measured cuBLAS burst peak), down 279 -> 181 us (1599), o 131 -> 78 us, QKV 154 -> 115 us; 7B gate/up 77 tokens 50 -> 38 us, INT8
 // 1500 tokens (expanded to fp16 first before) 411 + 74 -> 295 us.
 #include "gemm_common.cuh"

@@ -17,8 +17,9 @@
 //     of every rotation pair of a 128-wide head.  The warps of a CTA share an item's K groups, each with its next group's
 //     weights and activations in flight (70 KB an SM); their sums meet in shared memory, always in the same order.
 // Staging the activations as fragments in shared memory first was slower (gate/up of the 7B shape 27.6 us against 23.3: the
-// copy and its barrier stand before the first product), and so was not fetching them ahead (26.6).  At 3.1 TB/s (cold L2, with
-// the launch) the kernel issues 1.8 instructions per cycle: what is left is latency at the ends of items and issue.
+// copy and its barrier stand before the first product), and so was not fetching them ahead (26.6).  Started alone from a
+// cold L2 that is 3.1 TB/s, launch included; back to back with weights from memory 3.7 TB/s at 7168 x 14336 and 4.7 at 8192 x 28672
+// (one token, 14.9 and 26.6 us).  It issues 1.8 instructions per cycle: what is left is latency at the ends of items and issue.
 //
 // Epilogues: fp16 (+bias), SwiGLU, fp32 planes (K ranges, the consumer adds them), fused QKV (bias, rotate-half RoPE, K/V rows
 // into the paged cache).  Replaces for these passes the scalar GEMV kernels of the reference

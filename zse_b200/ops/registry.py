@@ -48,7 +48,8 @@ KERNEL_TABLE: Dict[str, Tuple[str, str]] = {
     "tiled_dequant_matmul_int8": ("gemm_w8_dec", "tcgen05, the INT4 decode kernel's pipeline with 8-bit chunks: weights "
                                                  "stay INT8 in memory and are dequantised into TMEM; passes of more "
                                                  "than 64 tokens take gemm_w8"),
-    "dequant_gemv_int4": ("gemm_w4", "M <= 8 streams the weights through registers (csrc/gemm_w4_small.cu) inside the same entry point"),
+    "dequant_gemv_int4": ("gemm_w4", "M <= 8 streams the weights through registers (csrc/gemm_w4_small.cu) inside the same entry point; "
+                                     "narrow and deep layers take a cluster along K"),
     "batched_dequant_gemv_int4": ("gemm_w4", "small batches take the narrow tensor-core tile"),
     "fused_gate_up_gemv_int4": ("gemm_w4", "epilogue 1: gate and up rows interleaved, activation applied in the epilogue"),
     "fp16_gemv": ("gemm_f16", ""),
