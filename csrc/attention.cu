@@ -58,7 +58,7 @@ __device__ __forceinline__ uint32_t tile_off(int row, int chunk) {
 }
 
 // ---- decode: how the work is cut -------------------------------------------------------------------------------------------
-// All 16-token tiles of all (sequence, kv head) items stand in one line, sequence by sequence.  With num_splits > 1 every CTA
+// All 16-token tiles of all (sequence, kv head) items stand in one line, sequence by sequence.  With num_splits > 2 every CTA
 // takes the same number of them, `per`, whatever items they belong to; an item that lies in several CTAs is merged from scratch
 // by attn_combine_kernel (at most num_splits - 1 pieces: `per` is raised for that if one sequence is very long).  The last of a
 // head's num_splits records in scratch says how many pieces there are.  That leaves nothing for two pieces, so with num_splits = 2
@@ -100,7 +100,7 @@ __device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
 //
 // With few sequences a launch is all start and end, and in a layer the instructions come from the L2 every time.  So everything but
 // the tile itself is kept short: one form of the cursors for any number of sequences (in lanes, no shared memory), loops that
-// stay loops, and one merge by all threads instead of two rounds between warps (60 KB of instructions before, 33 now).  One 7B
+// stay loops, and one merge by all threads instead of two rounds between warps (60 KB of instructions before, 35 now).  One 7B
 // sequence of 517 / 4000 tokens: 8.5 -> 7.5 / 12.9 -> 11.0 us with the merge of the pieces; 17 of 100 to 3000: 18.6 -> 16.9 us;
 // 14B, 64 of 128 to 2300: 69.6 -> 59.2 us cut, 57.1 -> 55.2 whole.
 template <int HD, bool EXT, int NB>
